@@ -441,7 +441,7 @@ int gpw_add_scalar(int dtype, int64_t n, double c, const void* x, void* y, gpw_s
 }
 
 static int reduce_common(int dtype, int op, int64_t nvec, int64_t n, const void* x, const void* y, double* out,
-                         gpw_stream stream, int ny = 1) {
+                         gpw_stream stream) {
   if (!valid_dtype(dtype) || nvec <= 0 || n <= 0 || !x || !out || nvec > 65535)
     return fail(GPW_EINVAL, "reduction: bad arguments");
   static thread_local SumScratch scratch;
@@ -451,7 +451,7 @@ static int reduce_common(int dtype, int op, int64_t nvec, int64_t n, const void*
   if (rc) return rc;
   GridSum gs = scratch.gs();
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = launch_reduce(dtype, op, nvec, n, x, y, gs, nblk, st, ny);
+  cudaError_t e = launch_reduce(dtype, op, nvec, n, x, y, gs, nblk, st);
   if (e != cudaSuccess) return cuda_fail(e, "reduction launch");
   e = cudaMemcpyAsync(out, gs.result, sizeof(double) * nvec * ncomp, cudaMemcpyDeviceToDevice, st);
   return e == cudaSuccess ? GPW_OK : cuda_fail(e, "reduction copy");
@@ -571,7 +571,15 @@ int gpw_dotc_pairs(int dtype, int64_t nx, int64_t ny, int64_t n, const void* x, 
                    gpw_stream stream) {
   if (!y) return fail(GPW_EINVAL, "null argument");
   if (nx <= 0 || ny <= 0 || nx * ny > 65535) return fail(GPW_EINVAL, "dotc_pairs: 1 <= nx * ny <= 65535");
-  return reduce_common(dtype, 2, nx * ny, n, x, y, out_dev, stream, (int)ny);
+  // a single pair reads each vector once: the plain reduction; several pairs
+  // share their vectors (one launch per pair read them from L2 again)
+  if (nx * ny == 1) return reduce_common(dtype, 2, 1, n, x, y, out_dev, stream);
+  if (!valid_dtype(dtype) || n <= 0 || !x || !out_dev) return fail(GPW_EINVAL, "reduction: bad arguments");
+  static thread_local Workspace scratch;
+  int rc = scratch.ensure(pair_scratch_bytes(dtype, nx, ny, n));
+  if (rc) return rc;
+  cudaError_t e = launch_pairs(dtype, nx, ny, n, x, y, (double*)scratch.ptr, out_dev, (cudaStream_t)stream);
+  return e == cudaSuccess ? GPW_OK : cuda_fail(e, "reduction launch");
 }
 
 }  // extern "C"
