@@ -6,6 +6,8 @@ end-to-end form) or a CUDA ``torch.Tensor`` (device-resident; zero copies).
 PyTorch is used only for device memory and the current CUDA stream; all
 arithmetic runs in libgpwgrid.so.
 """
+import math
+
 import numpy as np
 
 try:
@@ -21,13 +23,15 @@ _NP_TO_CODE = {np.dtype(np.float64): _lib.GPW_F64,
                np.dtype(np.complex64): _lib.GPW_C64}
 
 
-def _torch_maps():
-    return ({torch.float64: _lib.GPW_F64, torch.complex128: _lib.GPW_C128,
-             torch.float32: _lib.GPW_F32, torch.complex64: _lib.GPW_C64},
-            {np.dtype(np.float64): torch.float64,
-             np.dtype(np.complex128): torch.complex128,
-             np.dtype(np.float32): torch.float32,
-             np.dtype(np.complex64): torch.complex64})
+if torch is not None:
+    _TORCH_TO_NP = {torch.float64: np.dtype(np.float64),
+                    torch.complex128: np.dtype(np.complex128),
+                    torch.float32: np.dtype(np.float32),
+                    torch.complex64: np.dtype(np.complex64)}
+    _TORCH_TO_CODE = {t: _NP_TO_CODE[d] for t, d in _TORCH_TO_NP.items()}
+    _NP_TO_TORCH = {d: t for t, d in _TORCH_TO_NP.items()}
+    # the current stream's handle without a Stream object around it
+    _raw_stream = getattr(torch._C, '_cuda_getCurrentRawStream', None)
 
 
 def require_cuda():
@@ -42,50 +46,49 @@ def is_device(a):
 
 
 def stream():
-    return ctypes_stream(torch.cuda.current_stream())
-
-
-def ctypes_stream(s):
-    return s.cuda_stream
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def code_of(a):
     if is_device(a):
-        t2c, _ = _torch_maps()
-        return t2c[a.dtype]
+        return _TORCH_TO_CODE[a.dtype]
     return _NP_TO_CODE[np.dtype(a.dtype)]
 
 
 def np_dtype_of(a):
     if is_device(a):
-        return np.dtype({torch.float64: np.float64,
-                         torch.complex128: np.complex128,
-                         torch.float32: np.float32,
-                         torch.complex64: np.complex64}[a.dtype])
+        return _TORCH_TO_NP[a.dtype]
     return np.dtype(a.dtype)
+
+
+def grids_of(a):
+    """Number of grids in ``a`` (the product of its leading axes)."""
+    return math.prod(a.shape[:-3])
 
 
 def to_device(a):
     """CUDA tensor view of ``a`` (copied from the host for NumPy input)."""
-    require_cuda()
     if is_device(a):
         if not a.is_cuda:
+            require_cuda()
             raise ValueError('tensor must be on a CUDA device')
         if not a.is_contiguous():
             raise ValueError('array must be C-contiguous (as in the reference)')
         return a
+    require_cuda()
     a = np.asarray(a)
     if not a.flags.c_contiguous:
         a = np.ascontiguousarray(a)
-    _, np2t = _torch_maps()
-    if np.dtype(a.dtype) not in np2t:
+    if np.dtype(a.dtype) not in _NP_TO_TORCH:
         raise TypeError('unsupported dtype %s' % a.dtype)
     return torch.from_numpy(a).to('cuda', non_blocking=False)
 
 
 def empty_like_device(shape, dtype):
-    _, np2t = _torch_maps()
-    return torch.empty(tuple(shape), dtype=np2t[np.dtype(dtype)], device='cuda')
+    return torch.empty(tuple(shape), dtype=_NP_TO_TORCH[np.dtype(dtype)],
+                       device='cuda')
 
 
 def writeback(dst, src_dev):
@@ -106,5 +109,4 @@ def phases_arg(phase_cd):
     if phase_cd is None:
         return None, None
     p = np.ascontiguousarray(np.asarray(phase_cd, complex).reshape(3, 2))
-    buf = np.ascontiguousarray(p.view(np.float64).reshape(12))
-    return buf, buf.ctypes.data
+    return p, p.__array_interface__['data'][0]

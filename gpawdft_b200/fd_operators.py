@@ -111,7 +111,7 @@ class FDOperator:
         if code in (_lib.GPW_C128, _lib.GPW_C64) and phase_cd is not None:
             if np.asarray(phase_cd).shape != (3, 2):
                 raise ValueError('phase_cd must have shape (3, 2)')
-        nin = int(np.prod(in_xg.shape[:-3])) if len(in_xg.shape) > 3 else 1
+        nin = arrays.grids_of(in_xg)
         src = arrays.to_device(in_xg)
         dst = out_xg if arrays.is_device(out_xg) else None
         if dst is None:
@@ -149,7 +149,7 @@ class FDOperator:
         if code in (_lib.GPW_C128, _lib.GPW_C64) and phase_cd is not None:
             if np.asarray(phase_cd).shape != (3, 2):
                 raise ValueError('phase_cd must have shape (3, 2)')
-        nin = int(np.prod(in_xg.shape[:-3])) if len(in_xg.shape) > 3 else 1
+        nin = arrays.grids_of(in_xg)
         src = arrays.to_device(in_xg)
         pot = arrays.to_device(vt_g)
         dst = out_xg if arrays.is_device(out_xg) else None
@@ -184,7 +184,7 @@ class FDOperator:
         gpw_operator_apply_fused).  Device tensors."""
         self._check_grid(in_xg)
         code = arrays.code_of(in_xg)
-        nin = int(np.prod(in_xg.shape[:-3])) if len(in_xg.shape) > 3 else 1
+        nin = arrays.grids_of(in_xg)
         src = arrays.to_device(in_xg)
         dst = arrays.to_device(out_xg)
         pot = None if vt_g is None else arrays.to_device(vt_g)
@@ -229,7 +229,7 @@ class FDOperator:
         """r = A f - s and sum |r|^2 per grid (device tensors; new API)."""
         import torch
         code = arrays.code_of(f_g)
-        nin = int(np.prod(f_g.shape[:-3])) if len(f_g.shape) > 3 else 1
+        nin = arrays.grids_of(f_g)
         f = arrays.to_device(f_g)
         s = arrays.to_device(s_g)
         out = torch.empty(nin, dtype=torch.float64, device='cuda')

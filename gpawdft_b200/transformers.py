@@ -93,7 +93,7 @@ class _Transformer:
         code = arrays.code_of(input)
         if arrays.code_of(output) != code:
             raise ValueError('input and output dtypes differ')
-        nin = int(np.prod(xshape)) if xshape else 1
+        nin = arrays.grids_of(input)
         src = arrays.to_device(input)
         dst = output if arrays.is_device(output) else \
             arrays.empty_like_device(output.shape, output.dtype)
@@ -110,7 +110,7 @@ class _Transformer:
         """output = base - I(input) in one pass (interpolation only; device
         tensors; gpw_transformer_apply_subtract)."""
         code = arrays.code_of(input)
-        nin = int(np.prod(input.shape[:-3])) if len(input.shape) > 3 else 1
+        nin = arrays.grids_of(input)
         pbuf, pptr = arrays.phases_arg(phases)
         _lib.check(self._lib.gpw_transformer_apply_subtract(
             self._h, code, arrays.ptr(input), arrays.ptr(base),
