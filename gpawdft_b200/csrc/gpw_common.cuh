@@ -58,9 +58,49 @@ __device__ __forceinline__ float fmac(float c, float v, float a) { return fmaf(c
 __device__ __forceinline__ double2 fmac(double c, double2 v, double2 a) {
   return make_double2(fma(c, v.x, a.x), fma(c, v.y, a.y));
 }
+// (one packed instruction for both components: half the issue slots, the same
+// rounding as two fmaf)
 __device__ __forceinline__ float2 fmac(float c, float2 v, float2 a) {
-  return make_float2(fmaf(c, v.x, a.x), fmaf(c, v.y, a.y));
+  float2 r;
+  asm("{\n .reg .b64 c, v, a;\n mov.b64 c, {%2, %2};\n mov.b64 v, {%3, %4};\n mov.b64 a, {%5, %6};\n"
+      " fma.rn.f32x2 a, c, v, a;\n mov.b64 {%0, %1}, a;\n}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(c), "f"(v.x), "f"(v.y), "f"(a.x), "f"(a.y));
+  return r;
 }
+// Two points at once: a += c v, a += v and a = c v.  float32 pairs take one
+// packed instruction (half the issue slots, each half rounded as the scalar
+// instruction rounds).
+__device__ __forceinline__ void fma_pair(float c, float v0, float v1, float& a0, float& a1) {
+  const float2 r = fmac(c, make_float2(v0, v1), make_float2(a0, a1));
+  a0 = r.x;
+  a1 = r.y;
+}
+__device__ __forceinline__ void fma_pair(double c, double v0, double v1, double& a0, double& a1) {
+  a0 = fma(c, v0, a0);
+  a1 = fma(c, v1, a1);
+}
+__device__ __forceinline__ void add_pair(float v0, float v1, float& a0, float& a1) {
+  asm("{\n .reg .b64 v, a;\n mov.b64 v, {%2, %3};\n mov.b64 a, {%0, %1};\n add.rn.f32x2 a, a, v;\n"
+      " mov.b64 {%0, %1}, a;\n}\n"
+      : "+f"(a0), "+f"(a1)
+      : "f"(v0), "f"(v1));
+}
+__device__ __forceinline__ void add_pair(double v0, double v1, double& a0, double& a1) {
+  a0 += v0;
+  a1 += v1;
+}
+__device__ __forceinline__ void mul_pair(float c, float v0, float v1, float& a0, float& a1) {
+  asm("{\n .reg .b64 c, v;\n mov.b64 c, {%2, %2};\n mov.b64 v, {%3, %4};\n mul.rn.f32x2 v, c, v;\n"
+      " mov.b64 {%0, %1}, v;\n}\n"
+      : "=f"(a0), "=f"(a1)
+      : "f"(c), "f"(v0), "f"(v1));
+}
+__device__ __forceinline__ void mul_pair(double c, double v0, double v1, double& a0, double& a1) {
+  a0 = c * v0;
+  a1 = c * v1;
+}
+
 // round-to-nearest multiply then add, never contracted: x + (a * c) exactly as
 // the reference's `x += aa[offsets[c]] * coefs[c]` (c/bmgs/fd.c:42-43).
 __device__ __forceinline__ double mac_rn(double c, double v, double a) {

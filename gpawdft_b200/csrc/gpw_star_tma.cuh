@@ -364,24 +364,37 @@ __global__ void __launch_bounds__(TmaCfg<S, R, MODE, VAR>::NT, TmaCfg<S, R, MODE
             constexpr bool sweep = (MODE == MODE_JACOBI || MODE == MODE_JACOBI_ADD64 || MODE == MODE_JACOBI_SCALED_IN);
             // the in-plane sum in two independent chains (centre + axis 1,
             // axis 2) joined at the end: half the dependent-FMA latency
+            // (points in pairs: packed float32 instructions; a neighbour at an
+            // odd distance along axis 2 is no aligned pair)
             S p[VEC], pz[VEC];
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) {
-              p[e] = sweep ? S(0) : k.cc * c.v[e];
-              pz[e] = S(0);
+            for (int e = 0; e < VEC; e += 2) {
+              if constexpr (sweep)
+                p[e] = p[e + 1] = S(0);
+              else
+                mul_pair(k.cc, c.v[e], c.v[e + 1], p[e], p[e + 1]);
+              pz[e] = pz[e + 1] = S(0);
             }
 #pragma unroll
             for (int q = 1; q <= R; ++q) {
 #pragma unroll
-              for (int e = 0; e < VEC; ++e) {
-                p[e] = fma(k.cy[R + q], col[j + R + q].v[e], p[e]);
-                p[e] = fma(k.cy[R - q], col[j + R - q].v[e], p[e]);
-                pz[e] = fma(k.cz[R + q], nb[XL + e + q], pz[e]);
-                pz[e] = fma(k.cz[R - q], nb[XL + e - q], pz[e]);
+              for (int e = 0; e < VEC; e += 2) {
+                fma_pair(k.cy[R + q], col[j + R + q].v[e], col[j + R + q].v[e + 1], p[e], p[e + 1]);
+                fma_pair(k.cy[R - q], col[j + R - q].v[e], col[j + R - q].v[e + 1], p[e], p[e + 1]);
+                if (q % 2 == 0) {
+                  fma_pair(k.cz[R + q], nb[XL + e + q], nb[XL + e + 1 + q], pz[e], pz[e + 1]);
+                  fma_pair(k.cz[R - q], nb[XL + e - q], nb[XL + e + 1 - q], pz[e], pz[e + 1]);
+                } else {
+#pragma unroll
+                  for (int f = e; f < e + 2; ++f) {
+                    pz[f] = fma(k.cz[R + q], nb[XL + f + q], pz[f]);
+                    pz[f] = fma(k.cz[R - q], nb[XL + f - q], pz[f]);
+                  }
+                }
               }
             }
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) p[e] += pz[e];
+            for (int e = 0; e < VEC; e += 2) add_pair(pz[e], pz[e + 1], p[e], p[e + 1]);
             if constexpr (MODE == MODE_APPLY_EPI) {
               // local potential of this (in-range) plane: its part is output
               // plane pfirst + s's
@@ -398,11 +411,11 @@ __global__ void __launch_bounds__(TmaCfg<S, R, MODE, VAR>::NT, TmaCfg<S, R, MODE
             for (int m = 0; m < NR; ++m) {
               const int pm = (m + ph) % NR;
 #pragma unroll
-              for (int e = 0; e < VEC; ++e) {
+              for (int e = 0; e < VEC; e += 2) {
                 if (m == R)
-                  acc[j][pm].v[e] += p[e];
+                  add_pair(p[e], p[e + 1], acc[j][pm].v[e], acc[j][pm].v[e + 1]);
                 else
-                  acc[j][pm].v[e] = fma(k.cx[2 * R - m], c.v[e], acc[j][pm].v[e]);
+                  fma_pair(k.cx[2 * R - m], c.v[e], c.v[e + 1], acc[j][pm].v[e], acc[j][pm].v[e + 1]);
               }
             }
           }
