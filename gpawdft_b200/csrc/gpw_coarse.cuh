@@ -36,19 +36,16 @@ constexpr int CG_THREADS = 512;  // threads per CTA
 struct CoarseLevel {
   int n[3];
   int periodic[3];
-  int pts;                // elements per buffer: n0 n1 n2 (padded form: (n0+2)(n1+2)(n2+2))
+  int pts;                // elements per buffer: (n0+2)(n1+2)(n2+2)
   int base;               // element offset of the level's buffers: phi0, phi1, rho
   double cc;              // centre coefficient
   double cm[3], cp[3];    // neighbour coefficients at offsets -1 / +1 per axis
   int npre, npost;
   double w[CG_MAXW];      // pre-sweep weights, then post-sweep weights
-  int rpad0[3];           // restriction to the next level: low padding
-  int ipad0[3], iskip0[3];  // interpolation from the next level
 };
 
 struct CoarseArgs {
   int nl;                 // levels in the kernel (lc .. L)
-  int padded;             // zero boundaries everywhere: padded layout (see below)
   CoarseLevel lv[CG_MAXL];
   const void* rho;        // rho of level lc, engine layout
   GridView vrho;
@@ -57,135 +54,68 @@ struct CoarseArgs {
   const unsigned char* active;
 };
 
-__device__ __forceinline__ int cg_wrap(int i, int n, int periodic, bool& ok) {
-  ok = true;
-  if (i >= 0 && i < n) return i;
-  if (!periodic) {
-    ok = false;
-    return 0;
-  }
-  i %= n;
-  return i < 0 ? i + n : i;
-}
-
-template <typename S>
-__device__ __forceinline__ S cg_at(const S* buf, const CoarseLevel& L, int i0, int i1, int i2) {
-  bool o0, o1, o2;
-  i0 = cg_wrap(i0, L.n[0], L.periodic[0], o0);
-  i1 = cg_wrap(i1, L.n[1], L.periodic[1], o1);
-  i2 = cg_wrap(i2, L.n[2], L.periodic[2], o2);
-  return (o0 && o1 && o2) ? buf[(i0 * L.n[1] + i1) * L.n[2] + i2] : S(0);
-}
-
-__device__ __forceinline__ void cg_index(const CoarseLevel& L, int i, int& i0, int& i1, int& i2) {
-  i2 = i % L.n[2];
-  const int t = i / L.n[2];
-  i1 = t % L.n[1];
-  i0 = t / L.n[1];
-}
-
-// sum_{p != 0} c_p phi[x + o_p]
-template <typename S>
-__device__ __forceinline__ S cg_offdiag(const S* phi, const CoarseLevel& L, int i0, int i1, int i2) {
-  S av = (S)L.cm[2] * cg_at(phi, L, i0, i1, i2 - 1);
-  av = fmac((S)L.cp[2], cg_at(phi, L, i0, i1, i2 + 1), av);
-  av = fmac((S)L.cm[1], cg_at(phi, L, i0, i1 - 1, i2), av);
-  av = fmac((S)L.cp[1], cg_at(phi, L, i0, i1 + 1, i2), av);
-  av = fmac((S)L.cm[0], cg_at(phi, L, i0 - 1, i1, i2), av);
-  av = fmac((S)L.cp[0], cg_at(phi, L, i0 + 1, i1, i2), av);
-  return av;
-}
-
-// dst = (1 - w) src + (w / c0) (rho - sum_{p != 0} c_p src[x + o_p])   (c/bmgs/relax.c:62)
-template <typename S>
-__device__ __forceinline__ void cg_jacobi(const CoarseLevel& L, const S* src, S* dst, const S* rho, double wd) {
-  const S w = (S)wd, wc = w / (S)L.cc;
-  for (int i = threadIdx.x; i < L.pts; i += blockDim.x) {
-    int i0, i1, i2;
-    cg_index(L, i, i0, i1, i2);
-    const S av = cg_offdiag(src, L, i0, i1, i2);
-    dst[i] = (S(1) - w) * src[i] + wc * (rho[i] - av);
-  }
-  __syncthreads();
-}
-
-// r = A phi - rho
-template <typename S>
-__device__ __forceinline__ void cg_residual(const CoarseLevel& L, const S* phi, S* r, const S* rho) {
-  for (int i = threadIdx.x; i < L.pts; i += blockDim.x) {
-    int i0, i1, i2;
-    cg_index(L, i, i0, i1, i2);
-    const S av = cg_offdiag(phi, L, i0, i1, i2);
-    r[i] = fmac((S)L.cc, phi[i], av) - rho[i];
-  }
-  __syncthreads();
-}
-
-// rho_C = R r_F (K = 2) and phi_C = 0
-template <typename S>
-__device__ __forceinline__ void cg_restrict(const CoarseLevel& F, const S* r, const CoarseLevel& C, S* rho_c,
-                                            S* phi_c) {
-  for (int i = threadIdx.x; i < C.pts; i += blockDim.x) {
-    int I0, I1, I2;
-    cg_index(C, i, I0, I1, I2);
-    const int c0 = 1 + 2 * I0 - F.rpad0[0], c1 = 1 + 2 * I1 - F.rpad0[1], c2 = 1 + 2 * I2 - F.rpad0[2];
-    S y[3];
-#pragma unroll
-    for (int d0 = 0; d0 < 3; ++d0) {
-      S z[3];
-#pragma unroll
-      for (int d1 = 0; d1 < 3; ++d1)
-        z[d1] = r2(cg_at(r, F, c0 - 1 + d0, c1 - 1 + d1, c2 - 1), cg_at(r, F, c0 - 1 + d0, c1 - 1 + d1, c2),
-                   cg_at(r, F, c0 - 1 + d0, c1 - 1 + d1, c2 + 1));
-      y[d0] = r2(z[0], z[1], z[2]);
-    }
-    rho_c[i] = r2(y[0], y[1], y[2]);
-    phi_c[i] = S(0);
-  }
-  __syncthreads();
-}
-
-// dst = base - I e_C (K = 2)
-template <typename S>
-__device__ __forceinline__ S cg_interp_plane(const S* e, const CoarseLevel& C, int u0, int u1, int u2, int e1,
-                                             int e2) {
-  S z0 = cg_at(e, C, u0, u1, u2);
-  if (e2) z0 = i2h(z0, cg_at(e, C, u0, u1, u2 + 1));
-  if (!e1) return z0;
-  S z1 = cg_at(e, C, u0, u1 + 1, u2);
-  if (e2) z1 = i2h(z1, cg_at(e, C, u0, u1 + 1, u2 + 1));
-  return i2h(z0, z1);
-}
-
-template <typename S>
-__device__ __forceinline__ void cg_interp_sub(const CoarseLevel& F, const S* base, S* dst, const CoarseLevel& C,
-                                              const S* e) {
-  for (int i = threadIdx.x; i < F.pts; i += blockDim.x) {
-    int o0, o1, o2;
-    cg_index(F, i, o0, o1, o2);
-    const int t0 = o0 + F.iskip0[0], t1 = o1 + F.iskip0[1], t2 = o2 + F.iskip0[2];
-    const int u0 = (t0 >> 1) - F.ipad0[0], u1 = (t1 >> 1) - F.ipad0[1], u2 = (t2 >> 1) - F.ipad0[2];
-    S v = cg_interp_plane(e, C, u0, u1, u2, t1 & 1, t2 & 1);
-    if (t0 & 1) v = i2h(v, cg_interp_plane(e, C, u0 + 1, u1, u2, t1 & 1, t2 & 1));
-    dst[i] = base[i] - v;
-  }
-  __syncthreads();
-}
-
 // ---------------------------------------------------------------- padded form
-// When every level has zero boundaries, each level buffer is stored with a
-// one-point zero halo ((n0+2)(n1+2)(n2+2) elements, the halo never written):
-// neighbours sit at fixed offsets and need no bounds checks, and each thread
-// walks whole axis-0 columns by adding the plane stride, so no point pays an
-// index division.  `pts` then counts the padded elements.  The transfers
-// assume the zero-boundary K=2 tables: restriction pad 0 (fine centre
-// 2I + 1), interpolation pad 1 and skip 1 on every axis.
+// Each level buffer is stored with a one-point halo ((n0+2)(n1+2)(n2+2)
+// elements): neighbours sit at fixed offsets and need no bounds checks, and
+// each thread walks whole axis-0 columns by adding the plane stride, so no
+// point pays an index division.  `pts` counts the padded elements.  Along a
+// zero axis the halo is zero and never written; along a periodic axis the
+// thread that writes a boundary point also writes its images (edges and
+// corners included, which the transfers read), so no pass checks or wraps an
+// index.  (A layout without halo that wrapped every neighbour's index took
+// 64 us for the levels 10^3 and 5^3 of a periodic float64 V-cycle.)
+// The transfers take the K=2 tables of either boundary per axis: fine centre
+// of a coarse point 2I + fc (fc = 1 zero, 0 periodic), and coarse index
+// (o + fc) / 2 - fc of a fine point o.
 struct PadGeom {
   int n0, n1, n2;
   int sy, sz;  // padded row and plane strides
+  int fc0, fc1, fc2;   // 1: zero axis, 0: periodic
   __device__ __forceinline__ explicit PadGeom(const CoarseLevel& L)
-      : n0(L.n[0]), n1(L.n[1]), n2(L.n[2]), sy(L.n[2] + 2), sz((L.n[1] + 2) * (L.n[2] + 2)) {}
+      : n0(L.n[0]),
+        n1(L.n[1]),
+        n2(L.n[2]),
+        sy(L.n[2] + 2),
+        sz((L.n[1] + 2) * (L.n[2] + 2)),
+        fc0(L.periodic[0] ? 0 : 1),
+        fc1(L.periodic[1] ? 0 : 1),
+        fc2(L.periodic[2] ? 0 : 1) {}
   __device__ __forceinline__ int at(int i0, int i1, int i2) const { return (i0 + 1) * sz + (i1 + 1) * sy + i2 + 1; }
+  // the periodic boundaries point (i0, i1, i2) lies on: bits 2 axis (first
+  // point of the axis) and 2 axis + 1 (last)
+  __device__ __forceinline__ unsigned edges(int i0, int i1, int i2) const {
+    unsigned m = 0;
+    if (!fc0) m |= (i0 == 0 ? 1u : 0u) | (i0 == n0 - 1 ? 2u : 0u);
+    if (!fc1) m |= (i1 == 0 ? 4u : 0u) | (i1 == n1 - 1 ? 8u : 0u);
+    if (!fc2) m |= (i2 == 0 ? 16u : 0u) | (i2 == n2 - 1 ? 32u : 0u);
+    return m;
+  }
+  // v's periodic images in the halo, for a point at k on boundaries m (an
+  // axis of one point has both images)
+  template <typename S>
+  __device__ __forceinline__ void images(S* dst, int k, unsigned m, S v) const {
+    for (int e0 = 0; e0 < 3; ++e0) {
+      if (e0 && !(m & e0)) continue;
+      const int k0 = k + (e0 == 0 ? 0 : (e0 == 1 ? n0 * sz : -n0 * sz));
+      for (int e1 = 0; e1 < 3; ++e1) {
+        if (e1 && !((m >> 2) & e1)) continue;
+        const int k1 = k0 + (e1 == 0 ? 0 : (e1 == 1 ? n1 * sy : -n1 * sy));
+        dst[k1] = v;
+        if (m & 16u) dst[k1 + n2] = v;
+        if (m & 32u) dst[k1 - n2] = v;
+      }
+    }
+  }
+  // dst[k] = v, k = at(i0, i1, i2), and (PER: the level has a periodic axis)
+  // v's periodic images
+  template <bool PER, typename S>
+  __device__ __forceinline__ void put(S* dst, int i0, int i1, int i2, int k, S v) const {
+    dst[k] = v;
+    if constexpr (PER) {
+      const unsigned m = edges(i0, i1, i2);
+      if (m) images(dst, k, m, v);
+    }
+  }
 };
 
 // Walk the points of a padded level: each thread takes whole axis-0 columns
@@ -212,50 +142,108 @@ __device__ __forceinline__ void pg_points(const PadGeom& g, F body) {
   }
 }
 
-template <typename S>
+template <bool PER, typename S>
 __device__ __forceinline__ void pg_jacobi(const CoarseLevel& L, const S* __restrict__ src, S* __restrict__ dst,
                                           const S* __restrict__ rho, double wd) {
   const PadGeom g(L);
   const S w = (S)wd, wc = w / (S)L.cc;
   const S c0m = (S)L.cm[0], c0p = (S)L.cp[0], c1m = (S)L.cm[1], c1p = (S)L.cp[1], c2m = (S)L.cm[2],
           c2p = (S)L.cp[2];
-  pg_points(g, [&](int, int, int, int k) {
+  pg_points(g, [&](int i0, int i1, int i2, int k) {
     S av = c2m * src[k - 1];
     av = fmac(c2p, src[k + 1], av);
     av = fmac(c1m, src[k - g.sy], av);
     av = fmac(c1p, src[k + g.sy], av);
     av = fmac(c0m, src[k - g.sz], av);
     av = fmac(c0p, src[k + g.sz], av);
-    dst[k] = (S(1) - w) * src[k] + wc * (rho[k] - av);
+    g.template put<PER>(dst, i0, i1, i2, k, (S(1) - w) * src[k] + wc * (rho[k] - av));
   });
   __syncthreads();
 }
 
-template <typename S>
+// n sweeps on the buffers P, starting from P[c]; returns the buffer of the
+// result.  On levels of at most PG_U points a thread each thread finds its
+// points (index divisions, boundaries) once for all sweeps, whose passes are
+// then as short as their barrier: a sweep of a 10^3 or 7^3 level otherwise
+// spends most of its ~1 us on indices.
+constexpr int PG_U = 8;
+template <bool PER, typename S>
+__device__ __forceinline__ int pg_sweeps(const CoarseLevel& L, S* const (&P)[2], int c, const S* __restrict__ rho,
+                                         const double* w, int n) {
+  const PadGeom g(L);
+  const int ncol = g.n1 * g.n2, pts = ncol * g.n0, nt = blockDim.x;
+  if (n < 2 || ncol >= nt || pts > PG_U * nt) {
+    for (int s = 0; s < n; ++s, c = 1 - c) pg_jacobi<PER>(L, P[c], P[1 - c], rho, w[s]);
+    return c;
+  }
+  const S c0m = (S)L.cm[0], c0p = (S)L.cp[0], c1m = (S)L.cm[1], c1p = (S)L.cp[1], c2m = (S)L.cm[2],
+          c2p = (S)L.cp[2];
+  int k[PG_U];
+  unsigned m[PG_U];
+  S r[PG_U];
+#pragma unroll
+  for (int u = 0; u < PG_U; ++u) {
+    const int i = threadIdx.x + u * nt;
+    k[u] = -1;
+    m[u] = 0;
+    r[u] = S(0);
+    if (i < pts) {
+      const int i0 = i / ncol, q = i - i0 * ncol;
+      const int i1 = q / g.n2, i2 = q - i1 * g.n2;
+      k[u] = g.at(i0, i1, i2);
+      if (PER) m[u] = g.edges(i0, i1, i2);
+      r[u] = rho[k[u]];
+    }
+  }
+  for (int s = 0; s < n; ++s, c = 1 - c) {
+    const S* src = P[c];
+    S* dst = P[1 - c];
+    const S ws = (S)w[s], wc = ws / (S)L.cc;
+#pragma unroll
+    for (int u = 0; u < PG_U; ++u) {
+      if (u * nt >= pts) break;
+      if (k[u] < 0) continue;
+      const int q = k[u];
+      S av = c2m * src[q - 1];
+      av = fmac(c2p, src[q + 1], av);
+      av = fmac(c1m, src[q - g.sy], av);
+      av = fmac(c1p, src[q + g.sy], av);
+      av = fmac(c0m, src[q - g.sz], av);
+      av = fmac(c0p, src[q + g.sz], av);
+      const S v = (S(1) - ws) * src[q] + wc * (r[u] - av);
+      dst[q] = v;
+      if (PER && m[u]) g.images(dst, q, m[u], v);
+    }
+    __syncthreads();
+  }
+  return c;
+}
+
+template <bool PER, typename S>
 __device__ __forceinline__ void pg_residual(const CoarseLevel& L, const S* __restrict__ phi, S* __restrict__ r,
                                             const S* __restrict__ rho) {
   const PadGeom g(L);
   const S c0m = (S)L.cm[0], c0p = (S)L.cp[0], c1m = (S)L.cm[1], c1p = (S)L.cp[1], c2m = (S)L.cm[2],
           c2p = (S)L.cp[2], cc = (S)L.cc;
-  pg_points(g, [&](int, int, int, int k) {
+  pg_points(g, [&](int i0, int i1, int i2, int k) {
     S av = c2m * phi[k - 1];
     av = fmac(c2p, phi[k + 1], av);
     av = fmac(c1m, phi[k - g.sy], av);
     av = fmac(c1p, phi[k + g.sy], av);
     av = fmac(c0m, phi[k - g.sz], av);
     av = fmac(c0p, phi[k + g.sz], av);
-    r[k] = fmac(cc, phi[k], av) - rho[k];
+    g.template put<PER>(r, i0, i1, i2, k, fmac(cc, phi[k], av) - rho[k]);
   });
   __syncthreads();
 }
 
-// rho_C = R r_F and phi_C = 0 (zero boundaries: fine centre 2I + 1)
-template <typename S>
+// rho_C = R r_F and phi_C = 0 (its halo, written by an earlier pass, too)
+template <bool PER, typename S>
 __device__ __forceinline__ void pg_restrict(const CoarseLevel& F, const S* __restrict__ r, const CoarseLevel& C,
                                             S* __restrict__ rho_c, S* __restrict__ phi_c) {
   const PadGeom f(F), g(C);
   pg_points(g, [&](int I0, int I1, int I2, int k) {
-    const int kf = f.at(2 * I0 + 1, 2 * I1 + 1, 2 * I2 + 1);  // fine centre
+    const int kf = f.at(2 * I0 + f.fc0, 2 * I1 + f.fc1, 2 * I2 + f.fc2);  // fine centre
     S y[3];
 #pragma unroll
     for (int d0 = 0; d0 < 3; ++d0) {
@@ -268,12 +256,12 @@ __device__ __forceinline__ void pg_restrict(const CoarseLevel& F, const S* __res
       y[d0] = r2(z[0], z[1], z[2]);
     }
     rho_c[k] = r2(y[0], y[1], y[2]);
-    phi_c[k] = S(0);
+    g.template put<PER>(phi_c, I0, I1, I2, k, S(0));
   });
   __syncthreads();
 }
 
-// dst = base - I e_C (zero boundaries: skip0 = 1, pad0 = 1 on every axis)
+// dst = base - I e_C
 template <typename S>
 __device__ __forceinline__ S pg_interp_plane(const S* e, const PadGeom& g, int q, int e1, int e2) {
   S z0 = e[q];
@@ -284,27 +272,27 @@ __device__ __forceinline__ S pg_interp_plane(const S* e, const PadGeom& g, int q
   return i2h(z0, z1);
 }
 
-template <typename S>
+template <bool PER, typename S>
 __device__ __forceinline__ void pg_interp_sub(const CoarseLevel& F, const S* __restrict__ base, S* __restrict__ dst,
                                               const CoarseLevel& C, const S* __restrict__ e) {
   const PadGeom f(F), g(C);
   pg_points(f, [&](int o0, int o1, int o2, int k) {
-    // t = o + 1; coarse u = t / 2 - 1 (padded index u + 1 = t / 2), e = t & 1
-    const int t0 = o0 + 1, t1 = o1 + 1, t2 = o2 + 1;
+    // t = o + fc; coarse u = t / 2 - fc (padded index u + 1), e = t & 1
+    const int t0 = o0 + f.fc0, t1 = o1 + f.fc1, t2 = o2 + f.fc2;
     const int e1 = t1 & 1, e2 = t2 & 1;
-    const int q = (t0 >> 1) * g.sz + (t1 >> 1) * g.sy + (t2 >> 1);  // padded coarse index
+    const int q = g.at((t0 >> 1) - f.fc0, (t1 >> 1) - f.fc1, (t2 >> 1) - f.fc2);
     S v = pg_interp_plane(e, g, q, e1, e2);
     if (t0 & 1) v = i2h(v, pg_interp_plane(e, g, q + g.sz, e1, e2));
-    dst[k] = base[k] - v;
+    f.template put<PER>(dst, o0, o1, o2, k, base[k] - v);
   });
   __syncthreads();
 }
 
-template <typename S>
+template <bool PER, typename S>
 __device__ void coarse_vcycle_padded(const CoarseArgs& a, S* sm, int b) {
   const int nl = a.nl;
   int cur[CG_MAXL];
-  // zero every buffer once (the halos stay zero), then load rho of level 0
+  // zero every buffer once (zero-axis halos stay zero), then load rho of level 0
   int total = 0;
   for (int l = 0; l < nl; ++l) total = max(total, a.lv[l].base + 3 * a.lv[l].pts);
   for (int i = threadIdx.x; i < total; i += blockDim.x) sm[i] = S(0);
@@ -328,15 +316,14 @@ __device__ void coarse_vcycle_padded(const CoarseArgs& a, S* sm, int b) {
     const S* rho = sm + L.base + 2 * L.pts;
     int c = 0;
     if (l == nl - 1) {
-      for (int s = 0; s < L.npost; ++s, c = 1 - c) pg_jacobi(L, P[c], P[1 - c], rho, L.w[L.npre + s]);
-      cur[l] = c;
+      cur[l] = pg_sweeps<PER>(L, P, c, rho, L.w + L.npre, L.npost);
       break;
     }
-    for (int s = 0; s < L.npre; ++s, c = 1 - c) pg_jacobi(L, P[c], P[1 - c], rho, L.w[s]);
+    c = pg_sweeps<PER>(L, P, c, rho, L.w, L.npre);
     cur[l] = c;
-    pg_residual(L, P[c], P[1 - c], rho);
+    pg_residual<PER>(L, P[c], P[1 - c], rho);
     const CoarseLevel& C = a.lv[l + 1];
-    pg_restrict(L, P[1 - c], C, sm + C.base + 2 * C.pts, sm + C.base);
+    pg_restrict<PER>(L, P[1 - c], C, sm + C.base + 2 * C.pts, sm + C.base);
   }
   for (int l = nl - 2; l >= 0; --l) {
     const CoarseLevel& L = a.lv[l];
@@ -344,10 +331,8 @@ __device__ void coarse_vcycle_padded(const CoarseArgs& a, S* sm, int b) {
     S* P[2] = {sm + L.base, sm + L.base + L.pts};
     const S* rho = sm + L.base + 2 * L.pts;
     int c = cur[l];
-    pg_interp_sub(L, P[c], P[1 - c], C, sm + C.base + cur[l + 1] * C.pts);
-    c = 1 - c;
-    for (int s = 0; s < L.npost; ++s, c = 1 - c) pg_jacobi(L, P[c], P[1 - c], rho, L.w[L.npre + s]);
-    cur[l] = c;
+    pg_interp_sub<PER>(L, P[c], P[1 - c], C, sm + C.base + cur[l + 1] * C.pts);
+    cur[l] = pg_sweeps<PER>(L, P, 1 - c, rho, L.w + L.npre, L.npost);
   }
   {
     const CoarseLevel& L = a.lv[0];
@@ -362,71 +347,15 @@ __device__ void coarse_vcycle_padded(const CoarseArgs& a, S* sm, int b) {
   }
 }
 
-template <typename S>
-__global__ void __launch_bounds__(CG_THREADS, 1) coarse_vcycle_kernel(const CoarseArgs a) {
+template <typename S, bool PER>
+__global__ void __launch_bounds__(CG_THREADS, 1) coarse_vcycle_kernel(const __grid_constant__ CoarseArgs a) {
   pdl_wait();
   const int b = blockIdx.x;
   if (a.active && !a.active[b]) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   S* sm = reinterpret_cast<S*>(smem_raw);
-  if (a.padded) {
-    coarse_vcycle_padded(a, sm, b);
-    return;
-  }
-  const int nl = a.nl;
-  int cur[CG_MAXL];
-  {
-    const CoarseLevel& L = a.lv[0];
-    S* phi = sm + L.base;
-    S* rho = sm + L.base + 2 * L.pts;
-    const S* g = static_cast<const S*>(a.rho) + (int64_t)b * a.vrho.sb;
-    for (int i = threadIdx.x; i < L.pts; i += blockDim.x) {
-      int i0, i1, i2;
-      cg_index(L, i, i0, i1, i2);
-      rho[i] = g[(int64_t)i0 * a.vrho.s0 + (int64_t)i1 * a.vrho.s1 + i2];
-      phi[i] = S(0);
-    }
-    __syncthreads();
-  }
-  // descend
-  for (int l = 0; l < nl; ++l) {
-    const CoarseLevel& L = a.lv[l];
-    S* P[2] = {sm + L.base, sm + L.base + L.pts};
-    const S* rho = sm + L.base + 2 * L.pts;
-    int c = 0;
-    if (l == nl - 1) {
-      for (int s = 0; s < L.npost; ++s, c = 1 - c) cg_jacobi(L, P[c], P[1 - c], rho, L.w[L.npre + s]);
-      cur[l] = c;
-      break;
-    }
-    for (int s = 0; s < L.npre; ++s, c = 1 - c) cg_jacobi(L, P[c], P[1 - c], rho, L.w[s]);
-    cur[l] = c;
-    cg_residual(L, P[c], P[1 - c], rho);
-    const CoarseLevel& C = a.lv[l + 1];
-    cg_restrict(L, P[1 - c], C, sm + C.base + 2 * C.pts, sm + C.base);
-  }
-  // ascend
-  for (int l = nl - 2; l >= 0; --l) {
-    const CoarseLevel& L = a.lv[l];
-    const CoarseLevel& C = a.lv[l + 1];
-    S* P[2] = {sm + L.base, sm + L.base + L.pts};
-    const S* rho = sm + L.base + 2 * L.pts;
-    int c = cur[l];
-    cg_interp_sub(L, P[c], P[1 - c], C, sm + C.base + cur[l + 1] * C.pts);
-    c = 1 - c;
-    for (int s = 0; s < L.npost; ++s, c = 1 - c) cg_jacobi(L, P[c], P[1 - c], rho, L.w[L.npre + s]);
-    cur[l] = c;
-  }
-  {
-    const CoarseLevel& L = a.lv[0];
-    const S* phi = sm + L.base + cur[0] * L.pts;
-    S* g = static_cast<S*>(a.phi) + (int64_t)b * a.vphi.sb;
-    for (int i = threadIdx.x; i < L.pts; i += blockDim.x) {
-      int i0, i1, i2;
-      cg_index(L, i, i0, i1, i2);
-      g[(int64_t)i0 * a.vphi.s0 + (int64_t)i1 * a.vphi.s1 + i2] = phi[i];
-    }
-  }
+  coarse_vcycle_padded<PER>(a, sm, b);
+  pdl_trigger();
 }
 
 // ---------------------------------------------------------------- cluster top levels
@@ -565,7 +494,7 @@ __device__ __forceinline__ void slab_interp_sub(const CoarseLevel& F, int z0, co
 }
 
 template <typename S>
-__global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(const ClusterArgs a) {
+__global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(const __grid_constant__ ClusterArgs a) {
   namespace cg = cooperative_groups;
   pdl_wait();
   cg::cluster_group cl = cg::this_cluster();
@@ -618,20 +547,20 @@ __global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(c
   int c = 0;
   slab_exchange(cl, P[0], rank, np, npm, gs.sz);
   for (int s = t.first_done; s < T.npre; ++s, c = 1 - c) {
-    pg_jacobi(Ls, P[c], P[1 - c], rho, T.w[s]);
+    pg_jacobi<false>(Ls, P[c], P[1 - c], rho, T.w[s]);
     slab_exchange(cl, P[1 - c], rank, np, npm, gs.sz);
   }
-  pg_residual(Ls, P[c], P[1 - c], rho);
+  pg_residual<false>(Ls, P[c], P[1 - c], rho);
   slab_exchange(cl, P[1 - c], rank, np, npm, gs.sz);
   slab_restrict(Ls, P[1 - c], z0, y0, y1, U, rho2, gu.sz, gu.sy, y0, true);
   // ---- second level (phi = 0): pre-sweeps, residual, restriction into the third level (global)
   int d = 0;
   slab_exchange(cl, Q[0], rank, mp, mpm, gu.sz);  // (zeros: keeps the barrier sequence uniform)
   for (int s = 0; s < U.npre; ++s, d = 1 - d) {
-    pg_jacobi(Us, Q[d], Q[1 - d], rho2, U.w[s]);
+    pg_jacobi<false>(Us, Q[d], Q[1 - d], rho2, U.w[s]);
     slab_exchange(cl, Q[1 - d], rank, mp, mpm, gu.sz);
   }
-  pg_residual(Us, Q[d], Q[1 - d], rho2);
+  pg_residual<false>(Us, Q[d], Q[1 - d], rho2);
   slab_exchange(cl, Q[1 - d], rank, mp, mpm, gu.sz);
   const CoarseLevel& C = a.ca.lv[0];
   slab_restrict(Us, Q[1 - d], y0, y0 / 2, min(C.n[0], y1 / 2), C,
@@ -639,7 +568,7 @@ __global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(c
                 0, false);
   __threadfence();
   cl.sync();
-  if (rank == 0) coarse_vcycle_padded(a.ca, csm, b);
+  if (rank == 0) coarse_vcycle_padded<false>(a.ca, csm, b);
   __threadfence();
   cl.sync();
   {
@@ -659,7 +588,7 @@ __global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(c
   d = 1 - d;
   slab_exchange(cl, Q[d], rank, mp, mpm, gu.sz);
   for (int s = 0; s < U.npost; ++s, d = 1 - d) {
-    pg_jacobi(Us, Q[d], Q[1 - d], rho2, U.w[U.npre + s]);
+    pg_jacobi<false>(Us, Q[d], Q[1 - d], rho2, U.w[U.npre + s]);
     slab_exchange(cl, Q[1 - d], rank, mp, mpm, gu.sz);
   }
   // ---- top level: interpolation from the second level's slab (its halo planes included), post-sweeps
@@ -667,7 +596,7 @@ __global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(c
   c = 1 - c;
   slab_exchange(cl, P[c], rank, np, npm, gs.sz);
   for (int s = 0; s < T.npost; ++s, c = 1 - c) {
-    pg_jacobi(Ls, P[c], P[1 - c], rho, T.w[T.npre + s]);
+    pg_jacobi<false>(Ls, P[c], P[1 - c], rho, T.w[T.npre + s]);
     if (s + 1 < T.npost) slab_exchange(cl, P[1 - c], rank, np, npm, gs.sz);
   }
   {

@@ -11,6 +11,7 @@
 
 #include "gpw_blas.cuh"
 #include "gpw_coarse.cuh"
+#include "gpw_direct.cuh"
 #include "gpw_internal.h"
 #include "gpw_stencil.cuh"
 #include "gpw_transfer.cuh"
@@ -51,6 +52,32 @@ static void choose_chunks(int n0, int64_t tiles, int minz, int& zchunk, int& nch
 }
 
 // ------------------------------------------------------------------ stencils
+// Grids served by star_direct_kernel: all members together at most
+// DIRECT_BYTES of input (they stay in L2, and the marching kernels' chains of
+// planes cannot fill the chip).
+constexpr int64_t DIRECT_BYTES = 8 << 20;
+static bool direct_ok(const GridView& v, int64_t nbatch, size_t es) {
+  return (int64_t)v.n[0] * v.n[1] * v.n[2] * nbatch * (int64_t)es <= DIRECT_BYTES && nbatch <= 65535 &&
+         v.s0 <= INT32_MAX;
+}
+// its grid: 256 points of a plane and a run of planes per CTA, about 8 CTAs
+// per SM
+static dim3 direct_grid(const GridView& v, int64_t nbatch, int& zchunk) {
+  const int64_t bx = ((int64_t)v.n[1] * v.n[2] + DIRECT_NT - 1) / DIRECT_NT;
+  const int64_t tot = bx * v.n[0] * nbatch, want = 8LL * num_sms();
+  zchunk = (int)std::max<int64_t>(1, std::min<int64_t>(v.n[0], (tot + want - 1) / want));
+  return dim3((unsigned)bx, (v.n[0] + zchunk - 1) / zchunk, (unsigned)nbatch);
+}
+
+template <typename T, int R, int MODE>
+static cudaError_t run_direct(const StencilArgs& a0, const OpDesc& d, int nbatch, cudaStream_t st) {
+  StencilArgs a = a0;
+  const dim3 grid = direct_grid(a.vin, nbatch, a.zchunk);
+  a.nblk_seg = grid.x * grid.y;
+  return launch_pdl(star_direct_kernel<T, R, MODE>, grid, dim3(DIRECT_NT), 0, st, a,
+                    star_coefs_typed<typename EltTraits<T>::S>(d.sc));
+}
+
 template <typename T, int R, int MODE, bool EPI>
 static cudaError_t run_star_epi(const StencilArgs& a0, const OpDesc& d, int nbatch, cudaStream_t st) {
   using C = StarCfg<R, T>;
@@ -77,6 +104,7 @@ static cudaError_t run_star_epi(const StencilArgs& a0, const OpDesc& d, int nbat
 
 template <typename T, int R, int MODE>
 static cudaError_t run_star(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  if (direct_ok(a.vin, nbatch, sizeof(T))) return run_direct<T, R, MODE>(a, d, nbatch, st);
   if constexpr (MODE == MODE_APPLY) {
     if (a.pot || a.aux) return run_star_epi<T, R, MODE, true>(a, d, nbatch, st);
   }
@@ -241,7 +269,10 @@ int stencil_blocks_per_member(const OpDesc& d, int mode, const GridView& v, int 
   };
   int nblk;
   if (use_star) {
-    nblk = blocks(32, d.real ? GPW_STAR_TY : GPW_STAR_TY / 2, 2 * d.R + 2);  // complex128: half-height tiles
+    int zc;
+    const dim3 g = direct_grid(v, nbatch, zc);
+    nblk = direct_ok(v, nbatch, 4) ? (int)(g.x * g.y) : 0;
+    nblk = std::max(nblk, blocks(32, d.real ? GPW_STAR_TY : GPW_STAR_TY / 2, 2 * d.R + 2));  // complex128: half-height tiles
   } else {
     // the tile depends on the element size: the most CTAs over the op's types
     nblk = 0;
@@ -857,27 +888,23 @@ cudaError_t launch_cluster_vcycle(const ClusterArgs& a, size_t smem, int nbatch,
   return cudaLaunchKernelEx(&cfg, cluster_vcycle_kernel<float>, a);
 }
 
+template <typename S, bool PER>
+static cudaError_t run_coarse(const CoarseArgs& a, size_t smem, int nbatch, cudaStream_t st) {
+  static std::once_flag once;
+  static cudaError_t oe = cudaSuccess;
+  std::call_once(once, [] {
+    oe = cudaFuncSetAttribute(coarse_vcycle_kernel<S, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  });
+  if (oe != cudaSuccess) return oe;
+  return launch_pdl(coarse_vcycle_kernel<S, PER>, dim3(nbatch), dim3(CG_THREADS), smem, st, a);
+}
+
 cudaError_t launch_coarse(int dtype, const CoarseArgs& a, size_t smem, int nbatch, cudaStream_t st) {
   if (a.nl < 1 || a.nl > CG_MAXL || nbatch < 1 || smem > 200 * 1024) return cudaErrorInvalidValue;
-  if (dtype == GPW_F64) {
-    static std::once_flag once;
-    static cudaError_t oe = cudaSuccess;
-    std::call_once(once, [] {
-      oe = cudaFuncSetAttribute(coarse_vcycle_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                200 * 1024);
-    });
-    if (oe != cudaSuccess) return oe;
-    return launch_pdl(coarse_vcycle_kernel<double>, dim3(nbatch), dim3(CG_THREADS), smem, st, a);
-  } else if (dtype == GPW_F32) {
-    static std::once_flag once;
-    static cudaError_t oe = cudaSuccess;
-    std::call_once(once, [] {
-      oe = cudaFuncSetAttribute(coarse_vcycle_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                200 * 1024);
-    });
-    if (oe != cudaSuccess) return oe;
-    return launch_pdl(coarse_vcycle_kernel<float>, dim3(nbatch), dim3(CG_THREADS), smem, st, a);
-  }
+  bool per = false;
+  for (int c = 0; c < 3; ++c) per = per || a.lv[0].periodic[c];
+  if (dtype == GPW_F64) return per ? run_coarse<double, true>(a, smem, nbatch, st) : run_coarse<double, false>(a, smem, nbatch, st);
+  if (dtype == GPW_F32) return per ? run_coarse<float, true>(a, smem, nbatch, st) : run_coarse<float, false>(a, smem, nbatch, st);
   return cudaErrorInvalidValue;
 }
 
@@ -1069,11 +1096,11 @@ cudaError_t launch_transfer(const TrDesc& d, int dtype, const void* in, const Gr
     return dtype == GPW_F64 ? run_restrict_tma<double>(a, nbatch, st) : run_restrict_tma<float>(a, nbatch, st);
   if (d.k == 2 && (dtype == GPW_F64 || dtype == GPW_F32) && !interp && k2r_vec_ok(a)) {
     dim3 grid((vout.n[2] + 2 * K2V_TX - 1) / (2 * K2V_TX), (vout.n[1] + K2V_TY - 1) / K2V_TY, 1);
-    // ~8 CTAs of 256 threads per SM; chunks of at least 4 output planes
+    // ~8 CTAs of 256 threads per SM; chunks of at least 2 output planes
     const int64_t tiles = (int64_t)grid.x * grid.y * nbatch;
     const int64_t want = 8LL * num_sms();
     int64_t nc = std::max<int64_t>(1, (want + tiles - 1) / tiles);
-    nc = std::min<int64_t>(nc, std::max(1, vout.n[0] / 4));
+    nc = std::min<int64_t>(nc, std::max(1, vout.n[0] / 2));
     a.zchunk = (int)((vout.n[0] + nc - 1) / nc);
     a.nchunk = (vout.n[0] + a.zchunk - 1) / a.zchunk;
     grid.z = a.nchunk * nbatch;
@@ -1085,11 +1112,11 @@ cudaError_t launch_transfer(const TrDesc& d, int dtype, const void* in, const Gr
     return dtype == GPW_F64 ? run_interp_tma<double>(a, nbatch, st) : run_interp_tma<float>(a, nbatch, st);
   if (d.k == 2 && (dtype == GPW_F64 || dtype == GPW_F32) && interp && k2_vec_ok(a)) {
     dim3 grid((vout.n[2] + 4 * K2V_TX - 1) / (4 * K2V_TX), (vout.n[1] + K2V_TY - 1) / K2V_TY, 1);
-    // ~8 CTAs of 256 threads per SM; chunks of at least 8 output planes
+    // ~8 CTAs of 256 threads per SM; chunks of at least 2 output planes
     const int64_t tiles = (int64_t)grid.x * grid.y * nbatch;
     const int64_t want = 8LL * num_sms();
     int64_t nc = std::max<int64_t>(1, (want + tiles - 1) / tiles);
-    nc = std::min<int64_t>(nc, std::max(1, vout.n[0] / 8));
+    nc = std::min<int64_t>(nc, std::max(1, vout.n[0] / 2));
     a.zchunk = (int)((vout.n[0] + nc - 1) / nc);
     a.nchunk = (vout.n[0] + a.zchunk - 1) / a.zchunk;
     grid.z = a.nchunk * nbatch;
@@ -1099,7 +1126,9 @@ cudaError_t launch_transfer(const TrDesc& d, int dtype, const void* in, const Gr
   }
   if (d.k == 2 && (dtype == GPW_F64 || dtype == GPW_F32)) {
     dim3 grid((vout.n[2] + K2_TX - 1) / K2_TX, (vout.n[1] + K2_TY - 1) / K2_TY, 1);
-    choose_chunks(vout.n[0], (int64_t)grid.x * grid.y * nbatch, 4, a.zchunk, a.nchunk);
+    // single planes where even those leave SMs idle: a small grid's march is
+    // a chain of dependent loads
+    choose_chunks(vout.n[0], (int64_t)grid.x * grid.y * nbatch, interp ? 2 : 1, a.zchunk, a.nchunk);
     grid.z = a.nchunk * nbatch;
     const dim3 blk(K2_TX, K2_TY);
     if (dtype == GPW_F64) {

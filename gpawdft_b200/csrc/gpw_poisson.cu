@@ -433,10 +433,10 @@ const TrDesc* transformer_desc(const gpw_transformer* tr);
 // zero boundaries (padded form), 7-point Jacobi, every CTA owning planes of
 // both levels, and everything within one CTA's shared memory at two CTAs per
 // SM (so that all of a batch's clusters are resident together).
-static void setup_cluster_top(gpw_poisson* ps, bool padded, size_t es) {
+static void setup_cluster_top(gpw_poisson* ps, bool zero, size_t es) {
   ps->lt = -1;
   const int lc = ps->lc[1], nl = (int)ps->lv.size();
-  if (!ps->use_cluster || !padded || lc < 2 || lc + 1 >= nl || ps->relax_method != 2 || es != 4) return;
+  if (!ps->use_cluster || !zero || lc < 2 || lc + 1 >= nl || ps->relax_method != 2 || es != 4) return;
   const CoarseArgs& ca = ps->cargs[1];
   if (ca.nl < 2) return;
   const int lt = lc - 1;
@@ -474,9 +474,6 @@ static void setup_cluster_top(gpw_poisson* ps, bool padded, size_t es) {
   for (int a = 0; a < 3; ++a) {
     c.n[a] = L.v.n[a];
     c.periodic[a] = 0;
-    c.rpad0[a] = L.restr->pad[a][0];
-    c.ipad0[a] = L.interp->pad[a][0];
-    c.iskip0[a] = L.interp->skip[a][0];
   }
   c.pts = (int)slab;
   c.cc = d.sc.cc;
@@ -506,20 +503,25 @@ static void setup_coarse(gpw_poisson* ps, int p) {
   ps->lc[p] = nl;
   ps->csmem[p] = 0;
   if (ps->relax_method != 2) return;
-  // padded layout (zero halo) when no level of the hierarchy is periodic
-  // and the transfers have the zero-boundary K=2 tables
-  bool padded = true;
+  // the kernel's transfers are the K=2 ones of a zero or periodic axis; the
+  // cluster kernel takes zero boundaries only
+  bool zero = true;
+  auto tables_ok = [&](const Level& L) {
+    if (L.restr->k != 2 || L.interp->k != 2) return false;
+    for (int a = 0; a < 3; ++a) {
+      const int per = L.op->periodic[a] ? 1 : 0;
+      if (L.restr->pad[a][0] != per || L.interp->pad[a][0] != 1 - per || L.interp->skip[a][0] != 1 - per) return false;
+    }
+    return true;
+  };
   for (int l = 0; l < nl; ++l) {
     const Level& L = ps->lv[l];
-    for (int a = 0; a < 3; ++a) {
-      if (L.op->periodic[a]) padded = false;
-      if (l + 1 < nl && (L.restr->k != 2 || L.restr->pad[a][0] != 0 || L.interp->k != 2 ||
-                         L.interp->pad[a][0] != 1 || L.interp->skip[a][0] != 1))
-        padded = false;
-    }
+    for (int a = 0; a < 3; ++a)
+      if (L.op->periodic[a]) zero = false;
+    if (l + 1 < nl && !tables_ok(L)) zero = false;
   }
   auto buf_pts = [&](const Level& L) -> size_t {
-    return padded ? (size_t)(L.v.n[0] + 2) * (L.v.n[1] + 2) * (L.v.n[2] + 2) : (size_t)view_points(L.v);
+    return (size_t)(L.v.n[0] + 2) * (L.v.n[1] + 2) * (L.v.n[2] + 2);
   };
   size_t bytes = 0;
   int lc = nl;
@@ -528,6 +530,7 @@ static void setup_coarse(gpw_poisson* ps, int p) {
     const OpDesc& d = *L.op;
     if (!d.real || !d.star_jacobi || d.R != 1) break;
     if ((int)(L.wpre[p].size() + L.wpost[p].size()) > CG_MAXW) break;
+    if (l + 1 < nl && !tables_ok(L)) break;
     const size_t b = 3 * buf_pts(L) * es;
     if (bytes + b > budget) break;
     bytes += b;
@@ -537,7 +540,6 @@ static void setup_coarse(gpw_poisson* ps, int p) {
   CoarseArgs& ca = ps->cargs[p];
   ca = CoarseArgs{};
   ca.nl = nl - lc;
-  ca.padded = padded ? 1 : 0;
   int base = 0;
   for (int k = 0; k < ca.nl; ++k) {
     const Level& L = ps->lv[lc + k];
@@ -561,17 +563,10 @@ static void setup_coarse(gpw_poisson* ps, int p) {
     c.npost = (int)L.wpost[p].size();
     for (int i = 0; i < c.npre; ++i) c.w[i] = L.wpre[p][i];
     for (int i = 0; i < c.npost; ++i) c.w[c.npre + i] = L.wpost[p][i];
-    if (lc + k + 1 < nl) {
-      for (int a = 0; a < 3; ++a) {
-        c.rpad0[a] = L.restr->pad[a][0];
-        c.ipad0[a] = L.interp->pad[a][0];
-        c.iskip0[a] = L.interp->skip[a][0];
-      }
-    }
   }
   ps->lc[p] = lc;
   ps->csmem[p] = bytes;
-  if (p == 1) setup_cluster_top(ps, padded, es);
+  if (p == 1) setup_cluster_top(ps, zero, es);
 }
 
 int gpw_poisson_new(int nlevels, gpw_operator* const* operators, gpw_transformer* const* restrictors,
