@@ -42,7 +42,7 @@ EXPORTS = [
     'gpw_set_tma_variant', 'gpw_set_bloch_layout', 'gpw_bloch_launch_count',
     'gpw_set_restrict_layout', 'gpw_restrict_rows_launch_count',
     'gpw_poisson_set_device_loop', 'gpw_set_pdl', 'gpw_poisson_set_cluster',
-    'gpw_poisson_set_fusion',
+    'gpw_poisson_set_fusion', 'gpw_poisson_set_acceleration',
     'gpw_poisson_solve_many', 'gpw_poisson_last_latency',
     'gpw_poisson_profile_iteration', 'gpw_poisson_free',
     'gpw_nn_conv3', 'gpw_nn_wgrad_scratch', 'gpw_nn_conv3_wgrad',
@@ -146,6 +146,8 @@ _SIGS = {
     'gpw_set_pdl': (ctypes.c_int, [ctypes.c_int]),
     'gpw_poisson_set_cluster': (ctypes.c_int, [_vp, ctypes.c_int]),
     'gpw_poisson_set_fusion': (ctypes.c_int, [_vp, ctypes.c_int]),
+    'gpw_poisson_set_acceleration': (ctypes.c_int, [_vp, ctypes.c_double,
+                                                    ctypes.c_double]),
     'gpw_bloch_launch_count': (ctypes.c_int64, []),
     'gpw_set_restrict_layout': (ctypes.c_int, [ctypes.c_int]),
     'gpw_restrict_rows_launch_count': (ctypes.c_int64, []),

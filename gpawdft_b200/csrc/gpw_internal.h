@@ -92,12 +92,13 @@ cudaError_t launch_stencil(const OpDesc& d, int dtype, int mode, const void* in,
 // Fused defect-correction steps (TMA kernel; zero boundaries, 16-byte-pitched
 // engine buffers).  mode MODE_RESID_DC: in/rho float64, out (rhs) and out2
 // (first inner iterate) float32.  mode MODE_JACOBI_ADD64: in/rho float32,
-// out2 = float64 phi that receives the sweep's result.  Returns
+// out2 = float64 phi that receives the sweep's result times `step` (per
+// member; null: 1).  Returns
 // cudaErrorNotSupported when the TMA path does not apply.
 bool dc_fusable(const OpDesc& d);
 cudaError_t launch_stencil_dc(const OpDesc& d, int mode, const void* in, const GridView& v, void* out, void* out2,
                               const void* rho, int nbatch, double w, double w2, const unsigned char* active,
-                              const GridSum& gs, cudaStream_t st);
+                              const GridSum& gs, cudaStream_t st, const float* step = nullptr);
 
 // ---------------------------------------------------------------- transformer
 struct TrDesc {
@@ -141,7 +142,7 @@ cudaError_t tma_stencil_f32(int mode, int R, int var, const StencilArgs& a, int 
 // mode MODE_RESID_DC / MODE_JACOBI_ADD64 take the launch_stencil_dc arguments.
 cudaError_t tune_stencil(const OpDesc& d, int dtype, int mode, const void* in, const GridView& vin, void* out,
                          const GridView& vout, const void* rho, const GridView& vrho, void* out2, int nbatch,
-                         double w, const GridSum& gs, cudaStream_t st);
+                         double w, const GridSum& gs, cudaStream_t st, const float* step = nullptr);
 // Number of stencil choices tuned so far (the cache size).
 int tuned_stencil_count();
 

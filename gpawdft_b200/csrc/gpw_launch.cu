@@ -514,7 +514,7 @@ bool dc_fusable(const OpDesc& d) {
 
 cudaError_t launch_stencil_dc(const OpDesc& d, int mode, const void* in, const GridView& v, void* out, void* out2,
                               const void* rho, int nbatch, double w, double w2, const unsigned char* active,
-                              const GridSum& gs, cudaStream_t st) {
+                              const GridSum& gs, cudaStream_t st, const float* step) {
   if (!dc_fusable(d)) return cudaErrorNotSupported;
   const size_t es_in = (mode == MODE_RESID_DC) ? 8 : 4;
   if (!aligned16(in) || !aligned16(rho) || !aligned16(out2) || (out && !aligned16(out)) ||
@@ -531,6 +531,7 @@ cudaError_t launch_stencil_dc(const OpDesc& d, int mode, const void* in, const G
   a.c0 = d.coefs[0];
   a.active = active;
   a.gsum = gs;
+  a.step = step;
   if (mode != MODE_RESID_DC && mode != MODE_JACOBI_ADD64 && mode != MODE_JACOBI_SCALED_IN) return cudaErrorInvalidValue;
   const int dtype = (mode == MODE_RESID_DC) ? GPW_F64 : GPW_F32;
   const TmaChoice ch = tma_choice(dtype, d.R, mode, v, nbatch);
@@ -578,8 +579,9 @@ cudaError_t launch_resid_restrict(const OpDesc& d, const void* in, const void* r
 
 cudaError_t tune_stencil(const OpDesc& d, int dtype, int mode, const void* in, const GridView& vin, void* out,
                          const GridView& vout, const void* rho, const GridView& vrho, void* out2, int nbatch,
-                         double w, const GridSum& gs, cudaStream_t st) {
+                         double w, const GridSum& gs, cudaStream_t st, const float* step) {
   StencilArgs a{};
+  a.step = step;
   a.in = in;
   a.out = out;
   a.out2 = out2;

@@ -55,12 +55,33 @@ __device__ __forceinline__ int64_t global_ns() {
 // The convergence test of solve_neutral after each iteration.  A solve that
 // stops records the device clock in tdone[b]; with a conditional handle the
 // kernel also sets the condition of the graph's device-side while loop.
+// Step lengths of the outer iteration: the cyclic Chebyshev (Richardson)
+// iteration on a spectrum of the preconditioned operator within
+// [theta - delta, theta + delta] takes the reciprocals of the nodes of the
+// degree-ACCEL_M Chebyshev polynomial in turn.  (The three-term recurrence of
+// the same polynomials needs a direction stored and read on the fine grid,
+// ~8% of an iteration, to save less than one step in ten.)  A member whose
+// error grew takes plain steps from there on.
+constexpr int ACCEL_M = 5;
+struct OuterAccel {
+  float* step;      // per member: the next step's length; null: plain steps
+  double theta, delta;
+  // step k (from 0) of the cycle, the nodes ordered so that partial cycles
+  // damp the whole interval too
+  __device__ __forceinline__ void set(int b, int k) const {
+    if (!step) return;
+    const int order[ACCEL_M] = {2, 0, 4, 1, 3};
+    const int j = order[k % ACCEL_M];
+    step[b] = (float)(1.0 / (theta + delta * cospi((2 * j + 1) / (2.0 * ACCEL_M))));
+  }
+};
+
 __global__ void converge_update_kernel(int nbatch, const double* __restrict__ sumsq, double dv,
                                        const double* __restrict__ eps, const int* __restrict__ maxiter_p,
                                        double* __restrict__ err,
                                        int* __restrict__ niter, unsigned char* __restrict__ active,
                                        int* __restrict__ any_active, int64_t* __restrict__ tdone,
-                                       cudaGraphConditionalHandle cond, int use_cond) {
+                                       const OuterAccel acc, cudaGraphConditionalHandle cond, int use_cond) {
   __shared__ int any;
   const int maxiter = *maxiter_p;
   if (threadIdx.x == 0) any = 0;
@@ -68,6 +89,13 @@ __global__ void converge_update_kernel(int nbatch, const double* __restrict__ su
   for (int b = threadIdx.x; b < nbatch; b += blockDim.x) {
     if (!active[b]) continue;
     const double e = sumsq[b] * dv;
+    // (a step of exactly 1 marks a member that has left the accelerated steps)
+    if (acc.step) {
+      if (acc.step[b] != 1.f && (niter[b] == 1 || e <= err[b]))
+        acc.set(b, niter[b]);
+      else
+        acc.step[b] = 1.f;
+    }
     err[b] = e;
     // while iterate2(step) > eps and niter < maxiter: niter += 1
     if (e > eps[b] && niter[b] < maxiter) {
@@ -90,11 +118,13 @@ __global__ void stamp_kernel(int64_t* t) { *t = global_ns(); }
 // Per-solve state at the start of a solve; eps is read from the engine's
 // mapped pinned mailbox, so no copy engine is involved.
 __global__ void solve_setup_kernel(int nb, const double* __restrict__ h_eps, int maxiter, double* __restrict__ eps,
-                                   int* __restrict__ niter, unsigned char* __restrict__ active, int* maxiter_out) {
+                                   int* __restrict__ niter, unsigned char* __restrict__ active, int* maxiter_out,
+                                   const OuterAccel acc) {
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     eps[b] = h_eps[b];
     niter[b] = 1;
     active[b] = 1;
+    acc.set(b, 0);
   }
   if (threadIdx.x == 0) *maxiter_out = maxiter;
 }
@@ -163,6 +193,11 @@ struct gpw_poisson {
   bool use_cluster = true;
   bool use_rr = true;  // float32 form: level-0 residual restricted in the same launch
   bool use_rr_coarse = true;  // ... and the coarser levels' residuals
+  // Chebyshev acceleration of the float32 form's outer iteration: the
+  // spectrum taken for the V-cycle-preconditioned operator (hi <= lo: off),
+  // and the per-member step lengths
+  double accel_lo = 0.0, accel_hi = 0.0;
+  Workspace d_step;
   Workspace d_err, d_eps, d_niter, d_active, d_any, d_r64, d_gs_old, d_maxiter, d_tdone, d_t0;
   SumScratch sums;
   int* h_any = nullptr;  // pinned
@@ -229,12 +264,12 @@ struct Rec {
   }
   // one fused defect-correction stencil launch (or its tuning)
   void stencil_dc(const OpDesc& d, int mode, const void* in, const GridView& v, void* out, void* out2,
-                  const void* rho, double w, double w2, const GridSum& gs) {
+                  const void* rho, double w, double w2, const GridSum& gs, const float* step = nullptr) {
     if (tune)
       ok(tune_stencil(d, mode == MODE_RESID_DC ? GPW_F64 : GPW_F32, mode, in, v, out, v, rho, v, out2, nb,
-                      mode == MODE_RESID_DC ? w2 : w, gs, st));
+                      mode == MODE_RESID_DC ? w2 : w, gs, st, step));
     else
-      ok(launch_stencil_dc(d, mode, in, v, out, out2, rho, nb, w, w2, active, gs, st));
+      ok(launch_stencil_dc(d, mode, in, v, out, out2, rho, nb, w, w2, active, gs, st, step));
   }
 };
 
@@ -758,6 +793,11 @@ static int ensure_f32(gpw_poisson* ps) {
       return rc;
     for (Workspace* w : {&L.phi32[0], &L.phi32[1], &L.rho32, &L.res32}) cudaMemset(w->ptr, 0, w->bytes);
   }
+  if (ps->accel_hi > ps->accel_lo && fused_dc(ps) && !ps->d_step.ptr) {
+    const int rc = ps->d_step.ensure((size_t)ps->nbmax * sizeof(float));
+    if (rc) return rc;
+    cudaMemset(ps->d_step.ptr, 0, ps->d_step.bytes);  // (finite for a tuning pass before any solve)
+  }
   return GPW_OK;
 }
 
@@ -769,6 +809,17 @@ static bool fused_dc(const gpw_poisson* ps) {
   const Level& L0 = ps->lv[0];
   return ps->relax_method == 2 && ps->lv.size() >= 2 && !L0.wpre[1].empty() && !L0.wpost[1].empty() &&
          dc_fusable(*L0.op);
+}
+
+// The outer iteration's acceleration, where one is set and applies.
+static OuterAccel outer_accel(const gpw_poisson* ps) {
+  OuterAccel a{};
+  if (ps->accel_hi > ps->accel_lo && fused_dc(ps) && ps->d_step.ptr) {
+    a.step = (float*)ps->d_step.ptr;
+    a.theta = 0.5 * (ps->accel_lo + ps->accel_hi);
+    a.delta = 0.5 * (ps->accel_hi - ps->accel_lo);
+  }
+  return a;
 }
 
 // The float32 form's second level-0 pre-sweep reads the defect alone and
@@ -796,7 +847,7 @@ static cudaError_t record_iteration(gpw_poisson* ps, int nb, int prec, cudaStrea
                                               (const int*)ps->d_maxiter.ptr, (double*)ps->d_err.ptr,
                                               (int*)ps->d_niter.ptr, (unsigned char*)ps->d_active.ptr,
                                               (int*)ps->d_any.ptr, (int64_t*)ps->d_tdone.ptr,
-                                              cond ? *cond : cudaGraphConditionalHandle{}, cond ? 1 : 0);
+                                              prec == 1 ? outer_accel(ps) : OuterAccel{}, cond ? *cond : cudaGraphConditionalHandle{}, cond ? 1 : 0);
     r.ok(cudaGetLastError());
     r.tick("convergence update");
   };
@@ -854,7 +905,7 @@ static cudaError_t record_iteration(gpw_poisson* ps, int nb, int prec, cudaStrea
     cur = 1 - cur;
     cur = rec_relax(r, 0, cur, wpost.data(), (int)wpost.size() - 1, true);
     r.stencil_dc(*L0.op, MODE_JACOBI_ADD64, L0.phi32[cur].ptr, L0.v, nullptr, L0.phi[0].ptr, L0.rho32.ptr,
-                 wpost.back(), 0.0, GridSum{});
+                 wpost.back(), 0.0, GridSum{}, outer_accel(ps).step);
     r.tick("L0 f32 jacobi + phi64 update");
     r.stencil_dc(*L0.op, MODE_RESID_DC, L0.phi[0].ptr, L0.v, L0.rho32.ptr,
                  scaled_first(ps) ? nullptr : L0.phi32[0].ptr, L0.rho.ptr, 1.0, wpre[0], ps->sums.gs());
@@ -1017,7 +1068,8 @@ static int solve_prologue(gpw_poisson* ps, double* phi, const double* rho, int n
   Level& L0 = ps->lv[0];
   std::memcpy(ps->h_eps[slot], eps, (size_t)nb * 8);
   solve_setup_kernel<<<1, 128, 0, st>>>(nb, ps->m_eps[slot], maxiter, (double*)ps->d_eps.ptr, (int*)ps->d_niter.ptr,
-                                        (unsigned char*)ps->d_active.ptr, (int*)ps->d_maxiter.ptr);
+                                        (unsigned char*)ps->d_active.ptr, (int*)ps->d_maxiter.ptr,
+                                        precision == 1 ? outer_accel(ps) : OuterAccel{});
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = pitch_copy(L0.v, nb, phi, L0.v.n[2], (double*)L0.phi[0].ptr, L0.v.s1, st);
   if (e == cudaSuccess) e = pitch_copy(L0.v, nb, rho, L0.v.n[2], (double*)L0.rho.ptr, L0.v.s1, st);
@@ -1318,6 +1370,20 @@ extern "C" int gpw_poisson_set_inner_schedule(gpw_poisson* ps, const int* npre, 
     k += npost[l];
   }
   setup_coarse(ps, 1);
+  discard_f32_graphs(ps);
+  return GPW_OK;
+}
+
+// Chebyshev acceleration of the float32 form's outer iteration on a spectrum
+// of the V-cycle-preconditioned operator in [lo, hi] (hi <= lo: plain steps,
+// the default).  Applies to zero-boundary star Laplacians (the fused
+// defect-correction iteration).  Captured float32 graphs are discarded.
+extern "C" int gpw_poisson_set_acceleration(gpw_poisson* ps, double lo, double hi) {
+  if (!ps) return fail(GPW_EINVAL, "null argument");
+  if (!(lo >= 0.0) || !(hi >= 0.0) || (hi > lo && !(lo > 0.0)))
+    return fail(GPW_EINVAL, "set_acceleration: 0 < lo < hi, or hi <= lo to switch it off");
+  ps->accel_lo = lo;
+  ps->accel_hi = hi;
   discard_f32_graphs(ps);
   return GPW_OK;
 }

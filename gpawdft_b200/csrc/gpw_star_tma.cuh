@@ -321,6 +321,10 @@ __global__ void __launch_bounds__(TmaCfg<S, R, MODE, VAR>::NT, TmaCfg<S, R, MODE
         for (int m = 0; m < NR; ++m)
 #pragma unroll
           for (int e = 0; e < VEC; ++e) acc[j][m].v[e] = S(0);
+      float step = 1.f;  // JACOBI_ADD64: the outer step's length
+      if constexpr (MODE == MODE_JACOBI_ADD64) {
+        if (a.step) step = a.step[b];
+      }
       // RESID_RESTRICT: this thread's coarse points of the tile (tid + u NT)
       // and the in-plane restricted values of their last two fine planes
       constexpr int RK = C::RR ? (C::CX * C::CY + C::NT - 1) / C::NT : 1;
@@ -494,14 +498,14 @@ __global__ void __launch_bounds__(TmaCfg<S, R, MODE, VAR>::NT, TmaCfg<S, R, MODE
                     if (a.out2) stv_part<float, VEC>(ep, e1, nx);
                   }
                 } else if constexpr (MODE == MODE_JACOBI_ADD64) {
-                  // phi64 += e (the inner correction), e never stored
+                  // phi64 += step e (e the inner correction, never stored)
                   double* pp = static_cast<double*>(a.out2) + oidx;
                   const double* ap = asl + (yb + j) * C::TZ + VEC * tx;
 #pragma unroll
                   for (int h = 0; h < VEC; h += 2) {
                     Pack<double, 2> pv = ldv<double, 2>(ap + h);
-                    pv.v[0] += (double)res.v[h];
-                    pv.v[1] += (double)res.v[h + 1];
+                    pv.v[0] += (double)(step * res.v[h]);
+                    pv.v[1] += (double)(step * res.v[h + 1]);
                     if (h + 2 <= nx)
                       stv<double, 2>(pp + h, pv);
                     else

@@ -35,7 +35,7 @@ namespace gpw {
 // and writes the float32 defect rhs = -(A phi - rho) to `out` and the first
 // inner Jacobi iterate from zero, (w2 / c0) rhs, to `out2`, plus sum r^2;
 // JACOBI_ADD64 is a float32 Jacobi sweep whose result is added to the float64
-// array `out2` (phi += e) instead of being stored.  RESID_RESTRICT is a
+// array `out2` (phi += step e) instead of being stored.  RESID_RESTRICT is a
 // float32 residual that is not stored but restricted (K = 2, zero
 // boundaries) into the next level: rho_c to `out` and that level's first
 // Jacobi iterate from zero, (w2 / c0) rho_c with c0 the next level's
@@ -82,6 +82,7 @@ struct StencilArgs {
   int nblk_seg;     // CTAs per batch member
   void* out2;       // RESID_DC: first inner iterate (float); JACOBI_ADD64: float64 phi
   double w2;        // RESID_DC: Jacobi weight of that first inner sweep
+  const float* step;  // JACOBI_ADD64: per-member length of the outer step, phi64 += step e (null: 1)
   GridView vco;     // RESID_RESTRICT: the next level's view (out, out2)
   const void* pot;  // APPLY: optional local potential, one grid in the output's
                     // layout and the element's scalar type: out = A in + pot in

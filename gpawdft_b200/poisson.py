@@ -75,18 +75,25 @@ def jacobi_spectrum(op, lowest=False):
             axes.append(2 * np.pi * np.arange(n) / n)
         else:
             axes.append(np.pi * np.arange(1, n + 1) / (n + 1))
-    # the symbol is a sum of per-axis terms for star stencils; sample at
-    # most 64 modes per axis (it is smooth in theta)
+    # sample at most 64 modes per axis (the symbol is smooth in theta)
     axes = [a if len(a) <= 64 else
             np.unique(np.concatenate([a[::max(1, len(a) // 64)], a[-1:],
                                       a[:1]])) for a in axes]
-    t0, t1, t2 = np.meshgrid(*axes, indexing='ij')
-    c0 = None
-    sym = 0.0
-    for coef, o in zip(op.coef_p, op.offset_pc):
-        if not o.any():
-            c0 = coef if c0 is None else c0 + coef
-        sym = sym + coef * np.cos(o[0] * t0 + o[1] * t1 + o[2] * t2)
+    c0 = sum(c for c, o in zip(op.coef_p, op.offset_pc) if not o.any())
+    if all(np.count_nonzero(o) < 2 for o in op.offset_pc):
+        # a star's symbol is a sum of one function per axis
+        sym = c0
+        for c in range(3):
+            f = sum(coef * np.cos(o[c] * axes[c])
+                    for coef, o in zip(op.coef_p, op.offset_pc) if o[c])
+            shape = [1, 1, 1]
+            shape[c] = -1
+            sym = sym + np.reshape(f * np.ones(len(axes[c])), shape)
+    else:
+        t0, t1, t2 = np.meshgrid(*axes, indexing='ij')
+        sym = 0.0
+        for coef, o in zip(op.coef_p, op.offset_pc):
+            sym = sym + coef * np.cos(o[0] * t0 + o[1] * t1 + o[2] * t2)
     lam = sym / c0
     if lowest:
         nz = lam[lam > 1e-12 * lam.max()]
@@ -128,6 +135,38 @@ def inner_schedule(operators, fine=(2, 6.0), coarse=(3, 4.0), coarsest=8):
         npost.append(k)
         weights.extend(w + w[::-1])
     return npre, npost, weights
+
+
+def inner_spectrum(operators, fine=(2, 6.0), coarsest=8):
+    """Interval (lo, hi) of the eigenvalues of the V-cycle of
+    ``inner_schedule`` times A, on which the outer iteration is accelerated.
+
+    Below 1: the modes that the coarse grid does not see and the smoothing
+    damps least, one axis at half its highest frequency and the others
+    constant, keep P(lambda)^2 of the error (P: the level-0 sweeps'
+    Chebyshev polynomial, before and after).  Either side of 1: what the
+    coarsest level's sweeps leave of its error.  With nn=3 that is 0.79 for
+    equal spacings (Arnoldi on the cycle: 0.79 .. 1.04 on every grid from
+    32^3 to 40 x 72 x 104 points); the coarse operators' own error puts the
+    smooth modes up to 1.04.
+    """
+    op = operators[0]
+    hi = jacobi_spectrum(op)
+    k, ratio = fine
+    c0 = sum(c for c, o in zip(op.coef_p, op.offset_pc) if not o.any())
+    keep = 0.0
+    for axis in range(3):
+        lam = sum(c * np.cos(0.5 * np.pi * o[axis])
+                  for c, o in zip(op.coef_p, op.offset_pc)) / c0
+        p = np.prod([1.0 - w * lam
+                     for w in chebyshev_weights(k, hi / ratio, hi)])
+        keep = max(keep, float(p) ** 2)
+    top = jacobi_spectrum(operators[-1])
+    low = min(jacobi_spectrum(operators[-1], lowest=True), top)
+    # 1 / T_m((top + low) / (top - low)); a single mode is solved exactly
+    left = 0.0 if top - low < 1e-12 * top else \
+        1.0 / np.cosh(coarsest * np.arccosh((top + low) / (top - low)))
+    return 1.0 - max(keep, left) - 0.01, 1.0 + max(left, 0.045)
 
 
 def jacobi22_schedule(L, w=2.0 / 3.0, coarsest=8):
@@ -285,6 +324,9 @@ class FDPoissonSolver:
             a_w = (ctypes.c_double * len(ws))(*ws)
             _lib.check(lib.gpw_poisson_set_inner_schedule(h, a_pre, a_post,
                                                           a_w, len(ws)))
+            if self.inner == 'chebyshev':
+                _lib.check(lib.gpw_poisson_set_acceleration(
+                    h, *inner_spectrum(self.operators)))
 
     def set_device_loop(self, on=True):
         """Run the convergence loop on the device (default) or replay one

@@ -418,6 +418,16 @@ int gpw_poisson_set_cluster(gpw_poisson *ps, int on);
  * taking the stencil of the stored iterate).                              */
 int gpw_poisson_set_fusion(gpw_poisson *ps, int on);
 
+/* Chebyshev acceleration of the float32 form's outer (defect-correction)
+ * iteration (no counterpart in the reference): the spectrum of the inner
+ * V-cycle times A is taken to lie in [lo, hi], and the V-cycle's corrections
+ * are added with the step lengths of the cyclic Chebyshev iteration on it.  A
+ * solve whose error grows takes plain steps from there on.  Stopping test and
+ * precision are unchanged.  Zero-boundary star Laplacians; hi <= lo (the
+ * default) switches it off.  GPW_EINVAL for a null engine, a negative bound or
+ * lo = 0 < hi.                                                              */
+int gpw_poisson_set_acceleration(gpw_poisson *ps, double lo, double hi);
+
 /* Programmatic dependent launch of the V-cycle's kernels (no counterpart in
  * the reference): on = 1 (default) lets each stencil / transfer / coarse
  * kernel be dispatched while its predecessor drains (the kernel waits for
