@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS, 2) pair_mma_kernel(const PairAr
       }
 }
 
-// out[v] = sum over the parts of partial[part][v], in order within eight
+// out[v] = sum over the parts of partial[part][v], in order within 32
 // groups of parts and then over the groups, carrying each addition's rounding
 // error along (Knuth's two-sum): a plain sum of the ~300 parts was the largest
 // error of the result.
@@ -169,12 +169,14 @@ struct PairSum {
   }
 };
 
-__global__ void __launch_bounds__(256) pair_sum_kernel(int nv, int kparts, const double* __restrict__ partial,
+constexpr int PS_G = 32;  // groups of parts: a warp each (8 left the loads in a chain, 20 us)
+
+__global__ void __launch_bounds__(32 * PS_G) pair_sum_kernel(int nv, int kparts, const double* __restrict__ partial,
                                                        double* __restrict__ out) {
-  __shared__ PairSum red[8][32];
+  __shared__ PairSum red[PS_G][32];
   const int tx = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int v = blockIdx.x * 32 + tx;
-  const int p0 = kparts * g / 8, p1 = kparts * (g + 1) / 8;
+  const int p0 = kparts * g / PS_G, p1 = kparts * (g + 1) / PS_G;
   PairSum s{0.0, 0.0};
   if (v < nv) {
 #pragma unroll 8
@@ -184,7 +186,7 @@ __global__ void __launch_bounds__(256) pair_sum_kernel(int nv, int kparts, const
   __syncthreads();
   if (g == 0 && v < nv) {
 #pragma unroll
-    for (int i = 1; i < 8; ++i) {
+    for (int i = 1; i < PS_G; ++i) {
       s.add(red[i][tx].s);
       s.c += red[i][tx].c;
     }
@@ -270,7 +272,7 @@ cudaError_t launch_pairs(int dtype, int64_t nx, int64_t ny, int64_t n, const voi
   }
   if (e != cudaSuccess) return e;
   const int nv = (int)(nx * ny * (is_complex(dtype) ? 2 : 1));
-  pair_sum_kernel<<<(nv + 31) / 32, 256, 0, st>>>(nv, p.kparts, partial, out);
+  pair_sum_kernel<<<(nv + 31) / 32, 32 * PS_G, 0, st>>>(nv, p.kparts, partial, out);
   return cudaGetLastError();
 }
 
