@@ -51,6 +51,8 @@ static void choose_chunks(int n0, int64_t tiles, int minz, int& zchunk, int& nch
   nchunk = (n0 + zchunk - 1) / zchunk;
 }
 
+static int wave_chunks(int n, int64_t tiles, int warm, int64_t slots, int maxc);
+
 // ------------------------------------------------------------------ stencils
 // Grids served by star_direct_kernel: all members together at most
 // DIRECT_BYTES of input (they stay in L2, and the marching kernels' chains of
@@ -663,34 +665,50 @@ static cudaError_t tune_stencil_args(const OpDesc& d, int ldtype, int mode, cons
 }
 
 // ------------------------------------------------------------------ transfers
-template <typename T, int K>
-static cudaError_t run_restrict(TransferArgs a, int nbatch, cudaStream_t st) {
-  using C = RestrictCfg<T, K>;
-  dim3 grid((a.vout.n[2] + RS_OZ - 1) / RS_OZ, (a.vout.n[1] + RS_OY - 1) / RS_OY, 1);
-  choose_chunks(a.vout.n[0], (int64_t)grid.x * grid.y * nbatch, K, a.zchunk, a.nchunk);
+// One launch of a tile transfer kernel: shared-memory opt-in and its CTAs per
+// SM looked up once, axis 0 cut into the chunks (each paying `warm` planes
+// again) that fill whole waves.
+template <typename Kern>
+static cudaError_t run_transfer_tiles(Kern kern, std::once_flag& once, cudaError_t& oe, int& per_sm, dim3 block,
+                                      size_t smem, dim3 grid, int warm, int minz, TransferArgs a, int nbatch,
+                                      cudaStream_t st) {
+  std::call_once(once, [&] {
+    oe = smem_optin(kern, smem);
+    if (oe == cudaSuccess && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block.x * block.y, smem) !=
+                                 cudaSuccess)
+      per_sm = 1;
+  });
+  if (oe != cudaSuccess) return oe;
+  const int n0 = a.vout.n[0];
+  a.nchunk = wave_chunks(n0, (int64_t)grid.x * grid.y * nbatch, warm, (int64_t)std::max(1, per_sm) * num_sms(),
+                         std::max(1, n0 / minz));
+  a.zchunk = (n0 + a.nchunk - 1) / a.nchunk;
+  a.nchunk = (n0 + a.zchunk - 1) / a.zchunk;
   grid.z = a.nchunk * nbatch;
-  auto kern = restrict_kernel<T, K>;
-  static std::once_flag once;
-  cudaError_t e = cudaSuccess;
-  std::call_once(once, [&] { e = smem_optin(kern, C::smem); });
-  if (e != cudaSuccess) return e;
-  kern<<<grid, dim3(RS_OZ, RS_OY), C::smem, st>>>(a);
+  kern<<<grid, block, smem, st>>>(a);
   return cudaGetLastError();
 }
 
 template <typename T, int K>
-static cudaError_t run_interp(TransferArgs a, int nbatch, cudaStream_t st) {
-  using C = InterpCfg<T, K>;
-  dim3 grid((a.vout.n[2] + IP_OZ - 1) / IP_OZ, (a.vout.n[1] + IP_OY - 1) / IP_OY, 1);
-  choose_chunks(a.vout.n[0], (int64_t)grid.x * grid.y * nbatch, 2 * K, a.zchunk, a.nchunk);
-  grid.z = a.nchunk * nbatch;
-  auto kern = interpolate_kernel<T, K>;
+static cudaError_t run_restrict(const TransferArgs& a, int nbatch, cudaStream_t st) {
+  using C = RestrictCfg<T, K>;
   static std::once_flag once;
-  cudaError_t e = cudaSuccess;
-  std::call_once(once, [&] { e = smem_optin(kern, C::smem); });
-  if (e != cudaSuccess) return e;
-  kern<<<grid, dim3(IP_OZ, IP_OY), C::smem, st>>>(a);
-  return cudaGetLastError();
+  static cudaError_t oe = cudaSuccess;
+  static int per_sm = 1;
+  const dim3 grid((a.vout.n[2] + C::OZ - 1) / C::OZ, (a.vout.n[1] + C::OY - 1) / C::OY, 1);
+  return run_transfer_tiles(restrict_kernel<T, K>, once, oe, per_sm, dim3(C::OZ, C::OY), C::smem, grid, K - 1, 2, a,
+                            nbatch, st);
+}
+
+template <typename T, int K>
+static cudaError_t run_interp(const TransferArgs& a, int nbatch, cudaStream_t st) {
+  using C = InterpCfg<T, K>;
+  static std::once_flag once;
+  static cudaError_t oe = cudaSuccess;
+  static int per_sm = 1;
+  const dim3 grid((a.vout.n[2] + C::OZ - 1) / C::OZ, (a.vout.n[1] + C::OY - 1) / C::OY, 1);
+  return run_transfer_tiles(interpolate_kernel<T, K>, once, oe, per_sm, dim3(C::OZ, C::NTY), C::smem, grid,
+                            2 * (K - 1), 4, a, nbatch, st);
 }
 
 // Restriction layout: 0 = the launcher's choice, 1 = the tile kernel
@@ -803,7 +821,13 @@ static bool try_restrict_rows(const TransferArgs& a, int nbatch, cudaStream_t st
     return false;
   } else {
     const int force = g_restrict_force.load();
-    if (force == 1) return false;
+    // unpinned: complex data only (float64 32 x 96^3: the tile kernel takes
+    // 137 / 164 / 238 us at K = 4 / 6 / 8, this one 183 / 239 / 299), and of
+    // complex128 K = 2 and 6 (16 x 96^3: 86 / 180 us against 109 / 201; K = 4,
+    // 8: 133 / 261 against 126 / 261); complex64 32 x 96^3, K = 2 .. 8: 97 /
+    // 203 / 281 / 365 us against 168 / 216 / 310 / 411
+    const bool pick = sizeof(T) == 16 ? (K == 2 || K == 6) : EltTraits<T>::cpx;
+    if (force == 1 || (force == 0 && !pick)) return false;
     RowsPlan p;
     if (force == 3) {
       if (!rows_plan(a, K, sizeof(T), EltTraits<T>::cpx, 192, RowRestrictCfg<192>::MO, p)) return false;
@@ -840,14 +864,18 @@ static cudaError_t dispatch_transfer(const TransferArgs& a, int k, bool interp, 
   }
   if (interp) {
     switch (k) {
-      case 2: return run_interp<T, 2>(a, nbatch, st);
+      case 2:  // (complex past L2; else launch_transfer)
+        if constexpr (EltTraits<T>::cpx) return run_interp<T, 2>(a, nbatch, st);
+        break;
       case 4: return run_interp<T, 4>(a, nbatch, st);
       case 6: return run_interp<T, 6>(a, nbatch, st);
       case 8: return run_interp<T, 8>(a, nbatch, st);
     }
   } else {
     switch (k) {
-      case 2: return run_restrict<T, 2>(a, nbatch, st);
+      case 2:  // (complex past L2; else launch_transfer)
+        if constexpr (EltTraits<T>::cpx) return run_restrict<T, 2>(a, nbatch, st);
+        break;
       case 4: return run_restrict<T, 4>(a, nbatch, st);
       case 6: return run_restrict<T, 6>(a, nbatch, st);
       case 8: return run_restrict<T, 8>(a, nbatch, st);
@@ -1126,25 +1154,33 @@ cudaError_t launch_transfer(const TrDesc& d, int dtype, const void* in, const Gr
     if (dtype == GPW_F64) return launch_pdl(interpolate_k2_vec_kernel<double>, grid, blk, 0, st, a);
     return launch_pdl(interpolate_k2_vec_kernel<float>, grid, blk, 0, st, a);
   }
-  if (d.k == 2 && (dtype == GPW_F64 || dtype == GPW_F32)) {
+  // every other K = 2 transfer of real data, and complex ones that stay in L2
+  // (18^3 x 16 complex128: 6 us instead of the tile kernels' 16 - 30; at
+  // 72^3 x 16 these take 93 and 45 us against 70 and 36) unless a test pins
+  // their restriction kernel
+  const bool small = direct_ok(interp ? vout : vin, nbatch, elt_size(dtype));
+  if (d.k == 2 &&
+      (dtype == GPW_F64 || dtype == GPW_F32 || (small && (interp || g_restrict_force.load() == 0)))) {
     dim3 grid((vout.n[2] + K2_TX - 1) / K2_TX, (vout.n[1] + K2_TY - 1) / K2_TY, 1);
     // single planes where even those leave SMs idle: a small grid's march is
     // a chain of dependent loads
     choose_chunks(vout.n[0], (int64_t)grid.x * grid.y * nbatch, interp ? 2 : 1, a.zchunk, a.nchunk);
     grid.z = a.nchunk * nbatch;
     const dim3 blk(K2_TX, K2_TY);
-    if (dtype == GPW_F64) {
-      if (interp)
-        return launch_pdl(interpolate_k2_kernel<double>, grid, blk, 0, st, a);
-      else
-        return launch_pdl(restrict_k2_kernel<double>, grid, blk, 0, st, a);
-    } else {
-      if (interp)
-        return launch_pdl(interpolate_k2_kernel<float>, grid, blk, 0, st, a);
-      else
-        return launch_pdl(restrict_k2_kernel<float>, grid, blk, 0, st, a);
+    switch (dtype) {
+      case GPW_F64:
+        return interp ? launch_pdl(interpolate_k2_kernel<double>, grid, blk, 0, st, a)
+                      : launch_pdl(restrict_k2_kernel<double>, grid, blk, 0, st, a);
+      case GPW_F32:
+        return interp ? launch_pdl(interpolate_k2_kernel<float>, grid, blk, 0, st, a)
+                      : launch_pdl(restrict_k2_kernel<float>, grid, blk, 0, st, a);
+      case GPW_C128:
+        return interp ? launch_pdl(interpolate_k2_kernel<double2>, grid, blk, 0, st, a)
+                      : launch_pdl(restrict_k2_kernel<double2>, grid, blk, 0, st, a);
+      case GPW_C64:
+        return interp ? launch_pdl(interpolate_k2_kernel<float2>, grid, blk, 0, st, a)
+                      : launch_pdl(restrict_k2_kernel<float2>, grid, blk, 0, st, a);
     }
-    return cudaGetLastError();
   }
   switch (dtype) {
     case GPW_F64: return dispatch_transfer<double>(a, d.k, interp, nbatch, st);

@@ -9,7 +9,8 @@
 // an (axis-1, axis-2) output tile and marches along axis 0.  Each input plane
 // of the tile (with halo) is staged in shared memory by cp.async; the axis-2
 // pass and the axis-1 pass run in shared memory; the axis-0 pass gathers from
-// a per-thread register queue of the last planes' partial results.  Every 1D
+// a per-thread register queue of the last planes' partial results.  One CTA
+// barrier per step of the march.  Every 1D
 // pass evaluates the reference's expression in the reference's order with
 // unfused multiply / add, so results are bit-identical to the reference C.
 //
@@ -117,8 +118,10 @@ __device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ double2 radd(double2 a, double2 b) {
   return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
 }
+// (packed: one instruction for both components, each rounded as the scalar one)
 __device__ __forceinline__ float2 radd(float2 a, float2 b) {
-  return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+  add_pair(b.x, b.y, a.x, a.y);
+  return a;
 }
 __device__ __forceinline__ double rmul(double c, double a) { return __dmul_rn(c, a); }
 __device__ __forceinline__ float rmul(float c, float a) { return __fmul_rn(c, a); }
@@ -126,18 +129,21 @@ __device__ __forceinline__ double2 rmul(double c, double2 a) {
   return make_double2(__dmul_rn(c, a.x), __dmul_rn(c, a.y));
 }
 __device__ __forceinline__ float2 rmul(float c, float2 a) {
-  return make_float2(__fmul_rn(c, a.x), __fmul_rn(c, a.y));
+  float2 r;
+  mul_pair(c, a.x, a.y, r.x, r.y);
+  return r;
 }
 
 // K = 2 rules: 0.5 * (a0 + 0.5 * (a1 + a_1))   (c/bmgs/restrict.c:38-39)
 template <typename S>
 __device__ __forceinline__ S r2(S am, S a0, S ap) {
-  return rmul(S(0.5), radd(a0, rmul(S(0.5), radd(ap, am))));
+  using C = typename EltTraits<S>::S;
+  return rmul(C(0.5), radd(a0, rmul(C(0.5), radd(ap, am))));
 }
 // 0.5 * (a0 + a1)                 (c/bmgs/interpolate.c:33)
 template <typename S>
 __device__ __forceinline__ S i2h(S a0, S a1) {
-  return rmul(S(0.5), radd(a0, a1));
+  return rmul(typename EltTraits<S>::S(0.5), radd(a0, a1));
 }
 
 template <int K> struct TW;
@@ -186,193 +192,256 @@ __device__ __forceinline__ T interp_mid(const T* a, int st) {
 }
 
 // ------------------------------------------------------------------ restrict
-constexpr int RS_OZ = 32, RS_OY = 8;
-
+// A step takes the two fine planes of one coarse plane: the axis-2 pass of
+// step s (items of one staged row and MO adjacent outputs, the row's columns
+// read once; consecutive lanes take consecutive rows, whose odd pitch meets
+// no bank conflict) and the axis-1 / axis-0 pass of step s - 1 run between
+// the same two barriers, on two axis-2 buffers.  Of the 2K - 1 planes of an
+// output only the centre and the K at odd distance count, so a thread keeps
+// the last K even and K / 2 odd planes.
+// What bounds it: instruction issue and the float64 adds and multiplies of
+// the three unfused passes.
 template <typename T, int K>
 struct RestrictCfg {
-  static constexpr int H = 2 * RS_OY + 2 * K - 3;  // fine rows per plane tile
-  static constexpr int W = 2 * RS_OZ + 2 * K - 3;  // fine cols
-  static constexpr int NQ = 2 * K - 1;             // axis-0 taps span
-  static constexpr int NS = 3;                     // cp.async stages
-  static constexpr size_t smem = (size_t)NS * H * W * sizeof(T) + (size_t)H * RS_OZ * sizeof(T);
+  // tile of coarse points, one axis-1 item a thread; 16-byte elements of the
+  // wide stencils in half-width tiles (two CTAs per SM)
+  static constexpr int OZ = (sizeof(T) >= 16 && K >= 4) ? 16 : 32, OY = 8, NT = OZ * OY;
+  static constexpr int H = 2 * OY + 2 * K - 3;  // fine rows per plane tile
+  static constexpr int W = 2 * OZ + 2 * K - 3;  // fine cols (odd)
+  static constexpr int ZP = OZ + 1;             // axis-2 result pitch (odd)
+  static constexpr int MO = 4, NSEG = OZ / MO;  // axis-2 outputs per item
+  static constexpr int NS = 2;                  // stages of two planes
+  static constexpr size_t smem = (size_t)(NS * 2 * H * W + 2 * 2 * H * ZP) * sizeof(T);
 };
 
 template <typename T, int K>
-__global__ void __launch_bounds__(RS_OZ* RS_OY) restrict_kernel(const TransferArgs a) {
+__global__ void __launch_bounds__(RestrictCfg<T, K>::NT, 2) restrict_kernel(const TransferArgs a) {
   using C = RestrictCfg<T, K>;
-  constexpr int H = C::H, W = C::W, NQ = C::NQ, NS = C::NS;
+  using S = typename EltTraits<T>::S;
+  constexpr int H = C::H, W = C::W, ZP = C::ZP, MO = C::MO, NS = C::NS, KH = K / 2, NT = C::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* ring = reinterpret_cast<T*>(smem_raw);
-  T* zb = ring + NS * H * W;  // axis-2 pass result, H x RS_OZ
+  T* ring = reinterpret_cast<T*>(smem_raw);   // NS stages of two planes
+  T* zb = ring + NS * 2 * H * W;              // two buffers of two planes' axis-2 results
 
   const int b = blockIdx.z / a.nchunk, chunk = blockIdx.z - b * a.nchunk;
   if (a.active && !a.active[b]) return;
-  const int X0 = blockIdx.x * RS_OZ, Y0 = blockIdx.y * RS_OY;
+  const int X0 = blockIdx.x * C::OZ, Y0 = blockIdx.y * C::OY;
   const int I0 = chunk * a.zchunk, I1 = min(a.vout.n[0], I0 + a.zchunk);
   if (I0 >= I1) return;
   const T* in = static_cast<const T*>(a.in) + (int64_t)b * a.vin.sb;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + RS_OZ * ty;
-  // unpadded origin of the fine tile
-  const int ys = 2 * Y0 - a.pad0[1], xs = 2 * X0 - a.pad0[2];
-  // fine planes feeding outputs I0 .. I1-1: centre u(I) = K-1 + 2I - pad0
-  const int pfirst = K - 1 + 2 * I0 - a.pad0[0] - (K - 1);
-  const int plast = K - 1 + 2 * (I1 - 1) - a.pad0[0] + (K - 1);
-  const int nsteps = plast - pfirst + 1;
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + C::OZ * ty;
+  // fine planes feeding outputs I0 .. I1-1: step s takes planes pfirst + 2s
+  // and (not in the last step) pfirst + 2s + 1
+  const int pfirst = 2 * I0 - a.pad0[0];
+  const int nsteps = I1 - I0 + K - 1;
   const int Y = Y0 + ty, X = X0 + tx;
   const bool inside = Y < a.vout.n[1] && X < a.vout.n[2];
 
-  T q[NQ];
+  BoxLoader<T, H, W, NT> ld;
+  ld.init(a.vin, a.bc, 2 * Y0 - a.pad0[1], 2 * X0 - a.pad0[2]);
+  auto load = [&](int s) {
+    T* sl = ring + (s % NS) * 2 * H * W;
+    ld.load(sl, in, a.vin, a.bc, pfirst + 2 * s);
+    if (s + 1 < nsteps) ld.load(sl + H * W, in, a.vin, a.bc, pfirst + 2 * s + 1);
+  };
+  auto fix = [&](int s) {
+    if (!a.bc.use_phase) return;
+    T* sl = ring + (s % NS) * 2 * H * W;
+    ld.fix(sl, a.vin, a.bc, pfirst + 2 * s);
+    if (s + 1 < nsteps) ld.fix(sl + H * W, a.vin, a.bc, pfirst + 2 * s + 1);
+  };
+  T ev[K], od[KH];  // even planes 2(s-K+1) .. 2s, odd planes of the last K / 2 steps
 #pragma unroll
-  for (int i = 0; i < NQ; ++i) q[i] = zero<T>();
+  for (int i = 0; i < K; ++i) ev[i] = zero<T>();
+#pragma unroll
+  for (int i = 0; i < KH; ++i) od[i] = zero<T>();
 
-  BoxLoader<T, H, W, RS_OZ * RS_OY> ld;
-  ld.init(a.vin, a.bc, ys, xs);
 #pragma unroll
-  for (int st = 0; st < NS - 1; ++st) {
-    if (st < nsteps) ld.load(ring + st * H * W, in, a.vin, a.bc, pfirst + st);
+  for (int s = 0; s < NS; ++s) {
+    if (s < nsteps) load(s);
     cp_async_commit();
   }
-  for (int s = 0; s < nsteps; ++s) {
-    const int p = pfirst + s;
-    {
-      const int sn = s + NS - 1;
-      if (sn < nsteps) ld.load(ring + (sn % NS) * H * W, in, a.vin, a.bc, pfirst + sn);
-      cp_async_commit();
-    }
-    cp_async_wait<NS - 1>();
-    T* sl = ring + (s % NS) * H * W;
-    if (a.bc.use_phase) ld.fix(sl, a.vin, a.bc, p);
-    __syncthreads();
-    // axis-2 pass: zb[r][J] for all H rows
-    for (int idx = tid; idx < H * RS_OZ; idx += RS_OZ * RS_OY) {
-      const int r = idx / RS_OZ, J = idx - r * RS_OZ;
-      zb[idx] = restrict_1d<K>(sl + r * W + 2 * J + K - 1, 1);
-    }
-    __syncthreads();
-    // axis-1 pass for this thread's output column
-    const T v = restrict_1d<K>(zb + (2 * ty + K - 1) * RS_OZ + tx, RS_OZ);
+  cp_async_wait<NS - 1>();
+  fix(0);
+  __syncthreads();
+  for (int s = 0; s <= nsteps; ++s) {
+    if (s < nsteps) {
+      // axis-2 pass of both planes
+      const T* sl = ring + (s % NS) * 2 * H * W;
+      T* zs = zb + (s & 1) * 2 * H * ZP;
+      const int items = (s + 1 < nsteps ? 2 : 1) * H * C::NSEG;
+      for (int it = tid; it < items; it += NT) {
+        const int q = it / H, r = it - q * H;          // q: plane, segment
+        const int pl = q / C::NSEG, Ja = (q - pl * C::NSEG) * MO;
+        const T* rp = sl + (pl * H + r) * W + 2 * Ja;
+        T* zrow = zs + (pl * H + r) * ZP + Ja;
+        T w[MO + K - 1];
 #pragma unroll
-    for (int i = 0; i < NQ - 1; ++i) q[i] = q[i + 1];
-    q[NQ - 1] = v;
-    // plane p completes output I with u(I) + K - 1 == p
-    const int t = p - (K - 1) - (K - 1) + a.pad0[0];
-    if (s >= NQ - 1 && (t & 1) == 0) {
-      const int I = t >> 1;
-      if (I >= I0 && I < I1 && inside) {
-        const T o = restrict_1d<K>(q + (K - 1), 1);
-        static_cast<T*>(a.out)[(int64_t)b * a.vout.sb + (int64_t)I * a.vout.s0 + (int64_t)Y * a.vout.s1 + X] = o;
+        for (int t = 0; t < MO + K - 1; ++t) w[t] = rp[2 * t];
+#pragma unroll
+        for (int i = 0; i < MO; ++i) {
+          T sum = rp[2 * i + K - 1];
+#pragma unroll
+          for (int j = 0; j < KH; ++j)
+            sum = radd(sum, rmul((S)TW<K>::w(j), radd(w[i + KH + j], w[i + KH - 1 - j])));
+          zrow[i] = rmul(S(0.5), sum);
+        }
       }
     }
+    if (s >= 1) {
+      // axis-1 pass of step s - 1's planes, axis-0 sum of the output they complete
+      const int u = s - 1;
+      const T* zs = zb + (u & 1) * 2 * H * ZP + (2 * ty + K - 1) * ZP + tx;
+#pragma unroll
+      for (int i = 0; i < K - 1; ++i) ev[i] = ev[i + 1];
+      ev[K - 1] = restrict_1d<K>(zs, ZP);
+      const int t = u - (K - 1);
+      if (t >= 0 && inside) {
+        T sum = od[0];
+#pragma unroll
+        for (int j = 0; j < KH; ++j) sum = radd(sum, rmul((S)TW<K>::w(j), radd(ev[KH + j], ev[KH - 1 - j])));
+        static_cast<T*>(a.out)[(int64_t)b * a.vout.sb + (int64_t)(I0 + t) * a.vout.s0 + (int64_t)Y * a.vout.s1 + X] =
+            rmul(S(0.5), sum);
+      }
+#pragma unroll
+      for (int i = 0; i < KH - 1; ++i) od[i] = od[i + 1];
+      if (s < nsteps) od[KH - 1] = restrict_1d<K>(zs + H * ZP, ZP);
+    }
+    cp_async_wait<NS - 2>();
+    if (s + 1 < nsteps) fix(s + 1);
     __syncthreads();
+    if (s + NS < nsteps) load(s + NS);
+    cp_async_commit();
   }
 }
 
 // ------------------------------------------------------------------ interpolate
-constexpr int IP_OZ = 32, IP_OY = 8;
-
+// A step takes one coarse plane and yields two fine planes: the axis-2 pass
+// of step s (an item is one staged row and one coarse column: its copy and
+// its midpoint, from K values) and the axis-1 / axis-0 pass of step s - 1 run
+// between the same two barriers.  A thread owns PY adjacent fine rows of one
+// column, whose axis-1 pass reads K - 1 + PY / 2 values once, and keeps K
+// axis-0 values of each.
 template <typename T, int K>
 struct InterpCfg {
-  static constexpr int H = IP_OY / 2 + 1 + K;  // coarse rows per plane tile
-  static constexpr int W = IP_OZ / 2 + 1 + K;  // coarse cols
-  static constexpr int NQ = K;                 // axis-0 queue
+  static constexpr int OZ = 32, NTY = 8, NT = OZ * NTY;
+  // rows per thread, and CTAs per SM the registers must allow (4 rows of K
+  // axis-0 values do not fit two CTAs per SM for complex128 from K = 4 on
+  // and for 8-byte elements at K = 8)
+  static constexpr int PY = (sizeof(T) * K >= 64) ? 2 : 4;
+  static constexpr int MINB = (sizeof(T) * K >= 128) ? 1 : 2;
+  static constexpr int OY = NTY * PY, NM = PY / 2;
+  static constexpr int H = OY / 2 + K - 1;     // coarse rows per plane tile
+  static constexpr int W = OZ / 2 + K;         // coarse cols
   static constexpr int NS = 3;
-  static constexpr size_t smem = (size_t)NS * H * W * sizeof(T) + (size_t)H * IP_OZ * sizeof(T);
+  static constexpr size_t smem = (size_t)(NS * H * W + 2 * H * OZ) * sizeof(T);
 };
 
 template <typename T, int K>
-__global__ void __launch_bounds__(IP_OZ* IP_OY) interpolate_kernel(const TransferArgs a) {
+__global__ void __launch_bounds__(InterpCfg<T, K>::NT, (InterpCfg<T, K>::MINB)) interpolate_kernel(const TransferArgs a) {
   using C = InterpCfg<T, K>;
-  constexpr int H = C::H, W = C::W, NQ = C::NQ, NS = C::NS;
+  using S = typename EltTraits<T>::S;
+  constexpr int H = C::H, W = C::W, NS = C::NS, PY = C::PY, NM = C::NM, OZ = C::OZ, NT = C::NT;
   constexpr int base = K / 2 - 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* ring = reinterpret_cast<T*>(smem_raw);
-  T* zb = ring + NS * H * W;  // axis-2 pass result, H x IP_OZ
+  T* zb = ring + NS * H * W;  // axis-2 results, two buffers of H x OZ
 
   const int b = blockIdx.z / a.nchunk, chunk = blockIdx.z - b * a.nchunk;
   if (a.active && !a.active[b]) return;
-  const int X0 = blockIdx.x * IP_OZ, Y0 = blockIdx.y * IP_OY;
+  const int X0 = blockIdx.x * OZ, Y0 = blockIdx.y * C::OY;
   const int O0 = chunk * a.zchunk, O1 = min(a.vout.n[0], O0 + a.zchunk);
   if (O0 >= O1) return;
   const T* in = static_cast<const T*>(a.in) + (int64_t)b * a.vin.sb;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + IP_OZ * ty;
-  // coarse index i of a fine output o: o + skip0 = 2 i + e; centre c = base + i (padded)
-  // unpadded coarse coordinate of the centre: base + i - pad0.  Tile origin
-  // (unpadded) = centre of the first output minus (K/2 - 1).
-  const int iy0 = (Y0 + a.skip0[1]) >> 1, ix0 = (X0 + a.skip0[2]) >> 1;
-  const int ys = base + iy0 - a.pad0[1] - (K / 2 - 1);
-  const int xs = base + ix0 - a.pad0[2] - (K / 2 - 1);
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + OZ * ty;
+  // coarse index i of a fine output o: o + skip0 = 2 i + e, its centre the
+  // unpadded coarse point base + i - pad0; X0 and Y0 are even, so the tile's
+  // first outputs have i = X0 / 2, Y0 / 2 whatever the skip
+  const int sk1 = a.skip0[1], sk2 = a.skip0[2];
   const int i0f = (O0 + a.skip0[0]) >> 1, i0l = (O1 - 1 + a.skip0[0]) >> 1;
   const int pfirst = base + i0f - a.pad0[0] - (K / 2 - 1);
   const int plast = base + i0l - a.pad0[0] + K / 2;
   const int nsteps = plast - pfirst + 1;
-  const int oy = Y0 + ty, ox = X0 + tx;
-  const bool inside = oy < a.vout.n[1] && ox < a.vout.n[2];
-  // this thread's axis-1 position inside the coarse tile
-  const int ey = (oy + a.skip0[1]) & 1, ly = ((oy + a.skip0[1]) >> 1) - iy0 + (K / 2 - 1);
+  const int oy = Y0 + PY * ty, ox = X0 + tx;
+  const int rows = ox < a.vout.n[2] ? min(PY, a.vout.n[1] - oy) : 0;  // this thread's rows inside the grid
 
-  T q[NQ];
+  T q[PY][K];
 #pragma unroll
-  for (int i = 0; i < NQ; ++i) q[i] = zero<T>();
+  for (int j = 0; j < PY; ++j)
+#pragma unroll
+    for (int i = 0; i < K; ++i) q[j][i] = zero<T>();
+  T* outp = static_cast<T*>(a.out) + (int64_t)b * a.vout.sb + (int64_t)oy * a.vout.s1 + ox;
+  const T* basep = a.subtract ? static_cast<const T*>(a.base) + (int64_t)b * a.vbase.sb + (int64_t)oy * a.vbase.s1 + ox
+                              : nullptr;
 
-  BoxLoader<T, H, W, IP_OZ * IP_OY> ld;
-  ld.init(a.vin, a.bc, ys, xs);
+  BoxLoader<T, H, W, NT> ld;
+  ld.init(a.vin, a.bc, Y0 / 2 - a.pad0[1], X0 / 2 - a.pad0[2]);
 #pragma unroll
-  for (int st = 0; st < NS - 1; ++st) {
-    if (st < nsteps) ld.load(ring + st * H * W, in, a.vin, a.bc, pfirst + st);
+  for (int s = 0; s < NS; ++s) {
+    if (s < nsteps) ld.load(ring + s * H * W, in, a.vin, a.bc, pfirst + s);
     cp_async_commit();
   }
-  for (int s = 0; s < nsteps; ++s) {
-    const int p = pfirst + s;
-    {
-      const int sn = s + NS - 1;
-      if (sn < nsteps) ld.load(ring + (sn % NS) * H * W, in, a.vin, a.bc, pfirst + sn);
-      cp_async_commit();
-    }
-    cp_async_wait<NS - 1>();
-    T* sl = ring + (s % NS) * H * W;
-    if (a.bc.use_phase) ld.fix(sl, a.vin, a.bc, p);
-    __syncthreads();
-    // axis-2 pass: zb[r][x] for each fine output column x of the tile
-    for (int idx = tid; idx < H * IP_OZ; idx += IP_OZ * IP_OY) {
-      const int r = idx / IP_OZ, xl = idx - r * IP_OZ;
-      const int o = X0 + xl;
-      const int e = (o + a.skip0[2]) & 1, lx = ((o + a.skip0[2]) >> 1) - ix0 + (K / 2 - 1);
-      const T* rp = sl + r * W + lx;
-      zb[idx] = e ? interp_mid<K>(rp, 1) : rp[0];
-    }
-    __syncthreads();
-    // axis-1 pass for this thread's (oy, ox)
-    const T* cp = zb + ly * IP_OZ + tx;
-    const T v = ey ? interp_mid<K>(cp, IP_OZ) : cp[0];
+  cp_async_wait<NS - 1>();
+  if (a.bc.use_phase) ld.fix(ring, a.vin, a.bc, pfirst);
+  __syncthreads();
+  for (int s = 0; s <= nsteps; ++s) {
+    if (s < nsteps) {
+      // axis-2 pass: staged row r, coarse column li -> fine columns 2 li - skip
+      // (the copy) and 2 li + 1 - skip (the midpoint) of the tile
+      const T* sl = ring + (s % NS) * H * W;
+      T* zs = zb + (s & 1) * H * OZ;
+      for (int it = tid; it < H * (OZ / 2); it += NT) {
+        const int r = it / (OZ / 2), li = it - r * (OZ / 2);
+        const T* rp = sl + r * W + li;
+        T v[K];
 #pragma unroll
-    for (int i = 0; i < NQ - 1; ++i) q[i] = q[i + 1];
-    q[NQ - 1] = v;
-    // plane p (unpadded) = base + i - pad0 + d; outputs completed at this plane:
-    //  even o (e = 0) with centre plane == p          -> q[NQ-1]
-    //  odd  o (e = 1) with centre plane == p - K/2    -> taps q[NQ-1-K/2 - j .. ]
-    const int ic = p - base + a.pad0[0];  // i with centre at p
-    if (inside) {
-      T* outp = static_cast<T*>(a.out) + (int64_t)b * a.vout.sb + (int64_t)oy * a.vout.s1 + ox;
-      const T* basep = a.subtract ? static_cast<const T*>(a.base) + (int64_t)b * a.vbase.sb +
-                                        (int64_t)oy * a.vbase.s1 + ox
-                                  : nullptr;
-      {
-        const int o = 2 * ic - a.skip0[0];
-        if (o >= O0 && o < O1) {
-          const T val = q[NQ - 1];
-          outp[(int64_t)o * a.vout.s0] = a.subtract ? sub(basep[(int64_t)o * a.vbase.s0], val) : val;
-        }
+        for (int t = 0; t < K; ++t) v[t] = rp[t];
+        T* zp = zs + r * OZ + 2 * li - sk2;
+        if (2 * li - sk2 >= 0) zp[0] = v[base];
+        zp[1] = interp_mid<K>(v + base, 1);
       }
-      {
-        const int i = ic - K / 2;
-        const int o = 2 * i + 1 - a.skip0[0];
-        if (o >= O0 && o < O1 && s >= K - 1) {
-          const T val = interp_mid<K>(q + (NQ - 1 - K / 2), 1);
-          outp[(int64_t)o * a.vout.s0] = a.subtract ? sub(basep[(int64_t)o * a.vbase.s0], val) : val;
+      if (sk2)  // the copy at the tile's last column
+        for (int r = tid; r < H; r += NT) zs[r * OZ + OZ - 1] = sl[r * W + OZ / 2 + base];
+    }
+    if (s >= 1) {
+      const int p = pfirst + s - 1;
+      const T* cp = zb + ((s - 1) & 1) * H * OZ + NM * ty * OZ + tx;
+      T col[K - 1 + NM];
+#pragma unroll
+      for (int i = 0; i < K - 1 + NM; ++i) col[i] = cp[i * OZ];
+      const int ic = p - base + a.pad0[0];  // i with its centre at p
+      const int oe = 2 * ic - a.skip0[0], oo = 2 * (ic - K / 2) + 1 - a.skip0[0];
+      const bool ste = oe >= O0 && oe < O1, sto = oo >= O0 && oo < O1 && s - 1 >= K - 1;
+#pragma unroll
+      for (int j = 0; j < PY; ++j) {
+        // axis-1 pass: rows alternate between copies and midpoints, starting
+        // with a copy (skip 0) or a midpoint (skip 1)
+        const T mid = interp_mid<K>(col + base + (j >> 1), 1);
+        T v;
+        if ((j & 1) == 0)
+          v = sk1 ? mid : col[base + (j >> 1)];
+        else
+          v = sk1 ? col[base + (j >> 1) + 1] : mid;
+#pragma unroll
+        for (int i = 0; i < K - 1; ++i) q[j][i] = q[j][i + 1];
+        q[j][K - 1] = v;
+        if (j < rows) {
+          // plane p completes the even output centred at p and the odd one
+          // whose last tap is p
+          const int64_t oj = (int64_t)j * a.vout.s1, bj = (int64_t)j * a.vbase.s1;
+          if (ste) outp[(int64_t)oe * a.vout.s0 + oj] = a.subtract ? sub(basep[(int64_t)oe * a.vbase.s0 + bj], v) : v;
+          if (sto) {
+            const T m = interp_mid<K>(q[j] + base, 1);
+            outp[(int64_t)oo * a.vout.s0 + oj] = a.subtract ? sub(basep[(int64_t)oo * a.vbase.s0 + bj], m) : m;
+          }
         }
       }
     }
+    cp_async_wait<NS - 2>();
+    if (a.bc.use_phase && s + 1 < nsteps) ld.fix(ring + ((s + 1) % NS) * H * W, a.vin, a.bc, pfirst + s + 1);
     __syncthreads();
+    if (s + NS < nsteps) ld.load(ring + (s % NS) * H * W, in, a.vin, a.bc, pfirst + s + NS);
+    cp_async_commit();
   }
 }
 

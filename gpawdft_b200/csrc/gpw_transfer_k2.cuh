@@ -1,5 +1,5 @@
-// Direct-evaluation restriction and interpolation for K = 2 (nn = 1) on real
-// grids -- the transfers of every multigrid level of the Poisson solver and of
+// Direct-evaluation restriction and interpolation for K = 2 (nn = 1): the
+// transfers of every multigrid level of the Poisson solver and of
 // the eigensolver preconditioner.
 //
 // The K = 2 operators touch 3 (restriction) or 2 (interpolation) input points
@@ -12,8 +12,10 @@
 // carrying the axis-0 partial results of the previous plane.  The in-plane
 // addresses and boundary handling of a column are resolved once per thread
 // (zero boundary: a zero weight on an out-of-grid input; periodic: the
-// wrapped index; real data carries no Bloch phase), so the march itself is
-// loads and arithmetic only.
+// wrapped index, and for complex data its Bloch phases, axis 0, then 1, then
+// 2, as the reference's chained halo copies apply them), so the march itself
+// is loads and arithmetic only.  The two scalar kernels serve every element
+// type; the vector and TMA kernels below are real-only.
 #pragma once
 #include <climits>
 
@@ -26,74 +28,103 @@ namespace gpw {
 constexpr int K2_TX = 32, K2_TY = 8;
 
 // Resolve index i along an axis: element offset (times stride) and a
-// validity flag (false: zero-boundary halo, value 0).
-__device__ __forceinline__ bool k2_axis(int i, int n, int periodic, int64_t stride, int64_t& off) {
-  int j, s;
-  if (!wrap_axis(i, n, periodic, j, s)) {
+// validity flag (false: zero-boundary halo, value 0); side as in wrap_axis.
+__device__ __forceinline__ bool k2_axis(int i, int n, int periodic, int64_t stride, int64_t& off, int& side) {
+  int j;
+  if (!wrap_axis(i, n, periodic, j, side)) {
     off = 0;
     return false;
   }
   off = (int64_t)j * stride;
   return true;
 }
-
-template <typename S>
-__device__ __forceinline__ S k2_ld(const S* __restrict__ p, bool ok) {
-  return ok ? __ldg(p) : S(0);
+__device__ __forceinline__ bool k2_axis(int i, int n, int periodic, int64_t stride, int64_t& off) {
+  int side;
+  return k2_axis(i, n, periodic, stride, off, side);
 }
 
 template <typename S>
+__device__ __forceinline__ S k2_ld(const S* __restrict__ p, bool ok) {
+  return ok ? __ldg(p) : zero<S>();
+}
+
+// A column's in-plane taps: N x N positions (axis 1, axis 2), their offsets,
+// and the sides of the periodic images among them.
+template <typename T, int N>
+struct K2Column {
+  int64_t off[N][N];
+  bool ok[N][N];
+  int s1[N], s2[N];
+  bool image = false;  // some tap is an image along axis 1 or 2
+  __device__ __forceinline__ K2Column(const TransferArgs& a, int c1, int c2) {
+#pragma unroll
+    for (int d1 = 0; d1 < N; ++d1) {
+      int64_t o1, o2;
+      const bool v1 = k2_axis(c1 + d1, a.vin.n[1], a.bc.periodic[1], a.vin.s1, o1, s1[d1]);
+#pragma unroll
+      for (int d2 = 0; d2 < N; ++d2) {
+        const bool v2 = k2_axis(c2 + d2, a.vin.n[2], a.bc.periodic[2], 1, o2, s2[d2]);
+        off[d1][d2] = o1 + o2;
+        ok[d1][d2] = v1 && v2;
+        image |= s1[d1] >= 0 || s2[d2] >= 0;
+      }
+    }
+  }
+  // tap (d1, d2) of a plane at `pl` (v0: the plane is inside the grid or an
+  // image; s0: its side)
+  __device__ __forceinline__ T at(const TransferArgs& a, const T* pl, bool v0, int s0, int d1, int d2) const {
+    T v = k2_ld(pl + off[d1][d2], v0 && ok[d1][d2]);
+    if constexpr (EltTraits<T>::cpx) {
+      if (a.bc.use_phase && (image || s0 >= 0)) {
+        if (s0 >= 0) v = phase_mul(a.bc.ph[0][s0], v);
+        if (s1[d1] >= 0) v = phase_mul(a.bc.ph[1][s1[d1]], v);
+        if (s2[d2] >= 0) v = phase_mul(a.bc.ph[2][s2[d2]], v);
+      }
+    }
+    return v;
+  }
+};
+
+template <typename T>
 __global__ void __launch_bounds__(K2_TX* K2_TY) restrict_k2_kernel(const TransferArgs a) {
+  using S = typename EltTraits<T>::S;
   pdl_wait();
   const int b = blockIdx.z / a.nchunk, chunk = blockIdx.z - b * a.nchunk;
   if (a.active && !a.active[b]) return;
   const int I2 = blockIdx.x * K2_TX + threadIdx.x, I1 = blockIdx.y * K2_TY + threadIdx.y;
   if (I1 >= a.vout.n[1] || I2 >= a.vout.n[2]) return;
   const int I0s = chunk * a.zchunk, I0e = min(a.vout.n[0], I0s + a.zchunk);
-  const S* __restrict__ in = static_cast<const S*>(a.in) + (int64_t)b * a.vin.sb;
-  S* __restrict__ out = static_cast<S*>(a.out) + (int64_t)b * a.vout.sb + (int64_t)I1 * a.vout.s1 + I2;
+  const T* __restrict__ in = static_cast<const T*>(a.in) + (int64_t)b * a.vin.sb;
+  T* __restrict__ out = static_cast<T*>(a.out) + (int64_t)b * a.vout.sb + (int64_t)I1 * a.vout.s1 + I2;
   // fine centres (unpadded): c = 1 + 2 I - pad0; taps c-1, c, c+1
-  const int c1 = 1 + 2 * I1 - a.pad0[1], c2 = 1 + 2 * I2 - a.pad0[2];
-  int64_t off[3][3];  // [axis-1 tap][axis-2 tap] in-plane element offsets
-  bool ok[3][3];
-#pragma unroll
-  for (int d1 = 0; d1 < 3; ++d1) {
-    int64_t o1, o2;
-    const bool v1 = k2_axis(c1 - 1 + d1, a.vin.n[1], a.bc.periodic[1], a.vin.s1, o1);
-#pragma unroll
-    for (int d2 = 0; d2 < 3; ++d2) {
-      const bool v2 = k2_axis(c2 - 1 + d2, a.vin.n[2], a.bc.periodic[2], 1, o2);
-      off[d1][d2] = o1 + o2;
-      ok[d1][d2] = v1 && v2;
-    }
-  }
-  auto Y = [&](int f0) -> S {
+  const K2Column<T, 3> col(a, 2 * I1 - a.pad0[1], 2 * I2 - a.pad0[2]);
+  auto Y = [&](int f0) -> T {
     int64_t o0;
-    const bool v0 = k2_axis(f0, a.vin.n[0], a.bc.periodic[0], a.vin.s0, o0);
-    const S* pl = in + o0;
-    S z[3];
+    int s0;
+    const bool v0 = k2_axis(f0, a.vin.n[0], a.bc.periodic[0], a.vin.s0, o0, s0);
+    const T* pl = in + o0;
+    T z[3];
 #pragma unroll
     for (int d1 = 0; d1 < 3; ++d1)
-      z[d1] = r2(k2_ld(pl + off[d1][0], v0 && ok[d1][0]), k2_ld(pl + off[d1][1], v0 && ok[d1][1]),
-                 k2_ld(pl + off[d1][2], v0 && ok[d1][2]));
+      z[d1] = r2(col.at(a, pl, v0, s0, d1, 0), col.at(a, pl, v0, s0, d1, 1), col.at(a, pl, v0, s0, d1, 2));
     return r2(z[0], z[1], z[2]);
   };
-  S* __restrict__ out2 =
-      a.out2 ? static_cast<S*>(a.out2) + (int64_t)b * a.vout.sb + (int64_t)I1 * a.vout.s1 + I2 : nullptr;
+  T* __restrict__ out2 =
+      a.out2 ? static_cast<T*>(a.out2) + (int64_t)b * a.vout.sb + (int64_t)I1 * a.vout.s1 + I2 : nullptr;
   const S wc = (S)a.w2 / (S)a.c02;
-  S ylo = Y(1 + 2 * I0s - a.pad0[0] - 1);
+  T ylo = Y(1 + 2 * I0s - a.pad0[0] - 1);
 #pragma unroll 2
   for (int I0 = I0s; I0 < I0e; ++I0) {
     const int c0 = 1 + 2 * I0 - a.pad0[0];
-    const S ym = Y(c0), yp = Y(c0 + 1);
-    const S v = r2(ylo, ym, yp);
+    const T ym = Y(c0), yp = Y(c0 + 1);
+    const T v = r2(ylo, ym, yp);
     out[(int64_t)I0 * a.vout.s0] = v;
-    if (out2) out2[(int64_t)I0 * a.vout.s0] = wc * v;
+    if (out2) out2[(int64_t)I0 * a.vout.s0] = scale(wc, v);
     ylo = yp;
   }
 }
 
-template <typename S>
+template <typename T>
 __global__ void __launch_bounds__(K2_TX* K2_TY) interpolate_k2_kernel(const TransferArgs a) {
   pdl_wait();
   const int b = blockIdx.z / a.nchunk, chunk = blockIdx.z - b * a.nchunk;
@@ -101,37 +132,25 @@ __global__ void __launch_bounds__(K2_TX* K2_TY) interpolate_k2_kernel(const Tran
   const int o2 = blockIdx.x * K2_TX + threadIdx.x, o1 = blockIdx.y * K2_TY + threadIdx.y;
   if (o1 >= a.vout.n[1] || o2 >= a.vout.n[2]) return;
   const int O0s = chunk * a.zchunk, O0e = min(a.vout.n[0], O0s + a.zchunk);
-  const S* __restrict__ in = static_cast<const S*>(a.in) + (int64_t)b * a.vin.sb;
-  S* __restrict__ out = static_cast<S*>(a.out) + (int64_t)b * a.vout.sb + (int64_t)o1 * a.vout.s1 + o2;
-  const S* __restrict__ base =
-      a.subtract ? static_cast<const S*>(a.base) + (int64_t)b * a.vbase.sb + (int64_t)o1 * a.vbase.s1 + o2
+  const T* __restrict__ in = static_cast<const T*>(a.in) + (int64_t)b * a.vin.sb;
+  T* __restrict__ out = static_cast<T*>(a.out) + (int64_t)b * a.vout.sb + (int64_t)o1 * a.vout.s1 + o2;
+  const T* __restrict__ base =
+      a.subtract ? static_cast<const T*>(a.base) + (int64_t)b * a.vbase.sb + (int64_t)o1 * a.vbase.s1 + o2
                  : nullptr;
   // per axis: o + skip0 = 2 i + e; coarse (unpadded) index u = i - pad0
   const int t1 = o1 + a.skip0[1], t2 = o2 + a.skip0[2];
-  const int u1 = (t1 >> 1) - a.pad0[1], e1 = t1 & 1;
-  const int u2 = (t2 >> 1) - a.pad0[2], e2 = t2 & 1;
-  int64_t off[2][2];
-  bool ok[2][2];
-#pragma unroll
-  for (int d1 = 0; d1 < 2; ++d1) {
-    int64_t q1, q2;
-    const bool v1 = k2_axis(u1 + d1, a.vin.n[1], a.bc.periodic[1], a.vin.s1, q1);
-#pragma unroll
-    for (int d2 = 0; d2 < 2; ++d2) {
-      const bool v2 = k2_axis(u2 + d2, a.vin.n[2], a.bc.periodic[2], 1, q2);
-      off[d1][d2] = q1 + q2;
-      ok[d1][d2] = v1 && v2;
-    }
-  }
-  auto Y = [&](int u0) -> S {
+  const int e1 = t1 & 1, e2 = t2 & 1;
+  const K2Column<T, 2> col(a, (t1 >> 1) - a.pad0[1], (t2 >> 1) - a.pad0[2]);
+  auto Y = [&](int u0) -> T {
     int64_t q0;
-    const bool v0 = k2_axis(u0, a.vin.n[0], a.bc.periodic[0], a.vin.s0, q0);
-    const S* pl = in + q0;
-    S z0 = k2_ld(pl + off[0][0], v0 && ok[0][0]);
-    if (e2) z0 = i2h(z0, k2_ld(pl + off[0][1], v0 && ok[0][1]));
+    int s0;
+    const bool v0 = k2_axis(u0, a.vin.n[0], a.bc.periodic[0], a.vin.s0, q0, s0);
+    const T* pl = in + q0;
+    T z0 = col.at(a, pl, v0, s0, 0, 0);
+    if (e2) z0 = i2h(z0, col.at(a, pl, v0, s0, 0, 1));
     if (!e1) return z0;
-    S z1 = k2_ld(pl + off[1][0], v0 && ok[1][0]);
-    if (e2) z1 = i2h(z1, k2_ld(pl + off[1][1], v0 && ok[1][1]));
+    T z1 = col.at(a, pl, v0, s0, 1, 0);
+    if (e2) z1 = i2h(z1, col.at(a, pl, v0, s0, 1, 1));
     return i2h(z0, z1);
   };
   // march over coarse planes u: fine outputs o = 2 (u + pad0) + e0 - skip0
@@ -139,18 +158,18 @@ __global__ void __launch_bounds__(K2_TX* K2_TY) interpolate_k2_kernel(const Tran
   // the next plane do not depend on this plane's stores, so they run ahead
   const int us = ((O0s + a.skip0[0]) >> 1) - a.pad0[0];
   const int ue = ((O0e - 1 + a.skip0[0]) >> 1) - a.pad0[0];
-  S ya = Y(us);
+  T ya = Y(us);
 #pragma unroll 2
   for (int u = us; u <= ue; ++u) {
-    const S yb = Y(u + 1);
+    const T yb = Y(u + 1);
     const int oe = 2 * (u + a.pad0[0]) - a.skip0[0];
     if (oe >= O0s && oe < O0e) {
       const int64_t q = (int64_t)oe * a.vout.s0;
-      out[q] = a.subtract ? base[(int64_t)oe * a.vbase.s0] - ya : ya;
+      out[q] = a.subtract ? sub(base[(int64_t)oe * a.vbase.s0], ya) : ya;
     }
     if (oe + 1 >= O0s && oe + 1 < O0e) {
-      const S mid = i2h(ya, yb);
-      out[(int64_t)(oe + 1) * a.vout.s0] = a.subtract ? base[(int64_t)(oe + 1) * a.vbase.s0] - mid : mid;
+      const T mid = i2h(ya, yb);
+      out[(int64_t)(oe + 1) * a.vout.s0] = a.subtract ? sub(base[(int64_t)(oe + 1) * a.vbase.s0], mid) : mid;
     }
     ya = yb;
   }
