@@ -23,7 +23,8 @@ namespace {
 
 // A tile layout: VEC points per lane, WPR warps spanning a row, NW warps
 // per CTA (TY = NW / WPR * PY rows), and the axis-0 chunking; vec == 0
-// stands for the cp.async kernel of gpw_stencil.cuh.
+// stands for the kernel of gpw_stencil.cuh / gpw_direct.cuh, vec == -py for
+// the whole-row kernel (gpw_rows.cuh) with py rows a thread.
 struct BlochChoice {
   int vec, wpr, nw;
   int nchunk;  // 0: wave model, < 0: model x -nchunk
@@ -243,13 +244,16 @@ void tune_export_bloch(std::string& out) {
 }
 
 // One "bloch ..." record back into the tuner; a layout that is not among
-// the shape's candidates (nor the cp.async kernel, vec 0) is refused.
+// the shape's candidates (nor the cp.async kernel, vec 0, nor the whole-row
+// kernel, vec < 0) is refused.
 bool tune_import_bloch(const int* f) {
   const int dtype = f[0], R = f[1];
   if (!valid_dtype(dtype) || R < 1 || R > 3 || f[3] <= 0 || f[4] <= 0 || f[5] <= 0 || f[6] <= 0) return false;
   const BlochChoice c{f[7], f[8], f[9], f[10]};
   if (c.nchunk < -8 || c.nchunk > 64) return false;
-  if (c.vec != 0) {
+  if (c.vec < 0) {
+    if (c.vec != -4 && !(c.vec == -2 && dtype == GPW_C128)) return false;
+  } else if (c.vec != 0) {
     GridView v{};
     v.n[0] = f[3];
     v.n[1] = f[4];
@@ -265,6 +269,11 @@ bool tune_import_bloch(const int* f) {
   std::lock_guard<std::mutex> lock(g_bloch_mu);
   g_bloch_tune[BlochKey{dtype, R, f[2], f[3], f[4], f[5], f[6]}] = c;
   return true;
+}
+
+int rows_pinned() {
+  const int f = g_bloch_force.load();
+  return f == 15 ? 4 : (f == 16 ? 2 : 0);
 }
 
 bool bloch_path_ok(const OpDesc& d, int dtype, const void* in, const GridView& vin, const void* out,
@@ -290,7 +299,8 @@ cudaError_t launch_bloch(const OpDesc& d, int dtype, const StencilArgs& sa, int 
   const std::vector<BlochChoice> cands = bloch_candidates(dtype, d.R, vout);
   if (cands.empty()) return cudaErrorInvalidValue;
   auto run = [&](const BlochChoice& c) {
-    return c.vec == 0 ? launch_apply_cpasync(d, dtype, sa, nbatch, st)
+    if (c.vec < 0 && rows_ok(d, dtype, sa, -c.vec)) return launch_rows(d, dtype, sa, nbatch, -c.vec, st);
+    return c.vec <= 0 ? launch_apply_cpasync(d, dtype, sa, nbatch, st)
                       : bloch_launch(dtype, d.R, c, in, vin, out, vout, nbatch, bc, d.sc, sa.pot, sa.aux,
                                      sa.aux_scale, st);
   };
@@ -322,7 +332,9 @@ cudaError_t launch_bloch(const OpDesc& d, int dtype, const StencilArgs& sa, int 
           c.nchunk = nc;
           trial.push_back(c);
         }
-      trial.push_back(BlochChoice{0, 0, 0, 0});  // the cp.async kernel
+      trial.push_back(BlochChoice{0, 0, 0, 0});  // the cp.async or direct kernel
+      for (int py : {2, 4})
+        if (rows_ok(d, dtype, sa, py)) trial.push_back(BlochChoice{-py, 0, 0, 0});
       for (const BlochChoice& c : trial) {
         {
           cudaError_t e = run(c);  // warm-up
@@ -364,8 +376,9 @@ cudaError_t launch_bloch(const OpDesc& d, int dtype, const StencilArgs& sa, int 
 
 // Pins the tile layout of the periodic / Bloch stencil kernel: the k-th
 // candidate layout of each shape (k >= 1; shapes with fewer candidates keep
-// the tuned one), 0 = the tuned choice.  Process-wide; for tests and tuning
-// studies.
+// the tuned one), 15 / 16 the whole-row kernel with 4 / 2 rows a thread
+// wherever it takes the grid, 0 = the tuned choice.  Process-wide; for tests
+// and tuning studies.
 extern "C" int gpw_set_bloch_layout(int k) {
   if (k < 0 || k > 16) return gpw::fail(GPW_EINVAL, "bloch layout index must be 0-16");
   gpw::g_bloch_force.store(k);

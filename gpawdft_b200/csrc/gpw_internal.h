@@ -260,6 +260,13 @@ bool bloch_path_ok(const OpDesc& d, int dtype, const void* in, const GridView& v
                    const GridView& vout, int nbatch);
 struct StencilArgs;
 cudaError_t launch_bloch(const OpDesc& d, int dtype, const StencilArgs& a, int nbatch, cudaStream_t st);
+// The whole-row star apply (gpw_rows.cuh) with py rows a thread (4; complex128
+// also 2): whether it takes the grid, and its launch.
+bool rows_ok(const OpDesc& d, int dtype, const StencilArgs& sa, int py);
+bool rows_bulk_ok(const StencilArgs& sa, size_t es, int nbatch);
+int rows_pinned();  // rows a thread a test has pinned the kernel to, or 0
+cudaError_t launch_rows(const OpDesc& d, int dtype, const StencilArgs& sa, int nbatch, int py, cudaStream_t st);
+cudaError_t launch_rows_f32(const OpDesc& d, int dtype, const StencilArgs& sa, int nbatch, cudaStream_t st);
 // The cp.async star / general kernel for an apply.
 cudaError_t launch_apply_cpasync(const OpDesc& d, int dtype, const StencilArgs& a, int nbatch, cudaStream_t st);
 

@@ -244,6 +244,12 @@ static cudaError_t dispatch_mode(const StencilArgs& a, const OpDesc& d, int nbat
 
 static bool star_radius_ok(int R) { return R >= 1 && R <= 4; }
 
+static bool star_has_axis0(const OpDesc& d) {
+  for (int i = 0; i <= 2 * d.R; ++i)
+    if (d.sc.cx[i] != 0.0) return true;
+  return false;
+}
+
 // The cp.async star / general kernel for an apply (the periodic TMA row
 // kernel's tuner times it beside its own layouts).
 cudaError_t launch_apply_cpasync(const OpDesc& d, int dtype, const StencilArgs& a, int nbatch, cudaStream_t st) {
@@ -457,6 +463,8 @@ cudaError_t launch_stencil(const OpDesc& d, int dtype, int mode, const void* in,
   a.c0 = d.coefs.empty() ? 1.0 : d.coefs[0];
   a.active = active;
   a.gsum = gs;
+  if (const int py = rows_pinned(); py && mode == MODE_APPLY && !active && rows_ok(d, dtype, a, py))
+    return launch_rows(d, dtype, a, nbatch, py, st);
   if (tma_path_ok(d, dtype, mode, in, vin, out, vout, rho, vrho, nbatch)) {
     // first launch of an untuned shape outside stream capture: tune it now
     // (apply / residual / Jacobi recompute their output from inputs they do
@@ -479,6 +487,11 @@ cudaError_t launch_stencil(const OpDesc& d, int dtype, int mode, const void* in,
   }
   if (mode == MODE_APPLY && !active && bloch_path_ok(d, dtype, in, vin, out, vout, nbatch))
     return launch_bloch(d, dtype, a, nbatch, st);
+  // no axis-0 terms (a gradient): the whole-row kernel, which then stages no
+  // halo planes and keeps no sums
+  if (mode == MODE_APPLY && !active && !pot && !aux && !direct_ok(a.vin, nbatch, elt_size(dtype)) &&
+      !star_has_axis0(d) && rows_ok(d, dtype, a, 4))
+    return launch_rows(d, dtype, a, nbatch, 4, st);
   OpDesc dd = d;
   if (!star_radius_ok(dd.R)) {
     dd.star = false;

@@ -205,6 +205,15 @@ __device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap* map
       : "memory");
 }
 
+// Bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned)
+// from global memory into this CTA's shared memory, completing on `bar`.
+__device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                   dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
 // SYM: equal coefficients at +q and -q on every axis (a Laplacian): 3R + 1
 // coefficients fit in uniform registers, where 6R + 1 are loaded again on
 // every plane.

@@ -53,15 +53,6 @@ struct RowRestrictArgs {
 
 constexpr int RR_NS = 3;  // ring stages: two planes in flight while one is read
 
-// Bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned)
-// from global memory into this CTA's shared memory, completing on `bar`.
-__device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                   dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
 template <int NT>
 struct RowRestrictCfg {
   static constexpr int MO = NT >= 384 ? 4 : 6;  // axis-2 outputs per item

@@ -453,7 +453,8 @@ int gpw_set_tma_variant(int variant, int nchunk);
  * has up to 4 candidate layouts (a warp per row with 4 or 8 warps per CTA;
  * for complex rows wider than a warp, one point a lane with several warps
  * per row); k >= 1 pins the k-th (shapes with fewer keep the tuned one),
- * 0 returns to the tuned choice.  Process-wide; for tests and tuning
+ * 15 / 16 pin the whole-row kernel with 4 / 2 rows a thread on every apply
+ * it takes (2 rows: complex128), 0 returns to the tuned choice.  Process-wide; for tests and tuning
  * studies.  GPW_EINVAL outside [0, 16].                                   */
 int gpw_set_bloch_layout(int k);
 
