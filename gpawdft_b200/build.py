@@ -17,7 +17,8 @@ LIB = os.path.join(HERE, 'libgpwgrid.so')
 SOURCES = ['gpw_api.cu', 'gpw_launch.cu', 'gpw_poisson.cu', 'gpw_noalloc.cu',
            'gpw_tma_f64.cu', 'gpw_tma_f32.cu', 'gpw_nn.cu',
            'gpw_bloch.cu', 'gpw_woperator.cu', 'gpw_pairs.cu',
-           'gpw_rows_f64.cu', 'gpw_rows_f32.cu']
+           'gpw_rows_f64.cu', 'gpw_rows_f32.cu', 'gpw_cells_f64.cu',
+           'gpw_cells_f32.cu', 'gpw_cells_cpx.cu']
 
 
 def nvcc_path():

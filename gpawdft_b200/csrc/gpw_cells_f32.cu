@@ -1,0 +1,10 @@
+// Cell-staged star stencil launches for float32 grids.
+#include "gpw_star_cells_launch.cuh"
+
+namespace gpw {
+
+cudaError_t launch_cells_f32(int mode, const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  return cells_real<float>(mode, a, d, nbatch, st);
+}
+
+}  // namespace gpw

@@ -10,9 +10,8 @@
 // one or two memory latencies.  Taken for the grids direct_ok (gpw_launch.cu)
 // names.
 //
-// Each output sums its terms in the order of the cp.async star kernel
-// (axis 0 below, then the in-plane sum, then axis 0 above), so results do
-// not depend on which of the two ran.
+// An output's in-plane terms are one chain (centre, axis 1, axis 2), as
+// c/bmgs/fd.c sums a plane; latency is hidden by the other threads.
 #pragma once
 #include "gpw_common.cuh"
 #include "gpw_reduce.cuh"

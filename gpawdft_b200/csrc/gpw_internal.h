@@ -266,6 +266,12 @@ bool rows_ok(const OpDesc& d, int dtype, const StencilArgs& sa, int py);
 bool rows_bulk_ok(const StencilArgs& sa, size_t es, int nbatch);
 int rows_pinned();  // rows a thread a test has pinned the kernel to, or 0
 cudaError_t launch_rows(const OpDesc& d, int dtype, const StencilArgs& sa, int nbatch, int py, cudaStream_t st);
+// The cell-staged star stencil (gpw_star_cells.cuh): apply, residual and Jacobi
+// on real grids, applies on complex ones.
+cudaError_t launch_cells_f64(int mode, const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st);
+cudaError_t launch_cells_f32(int mode, const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st);
+cudaError_t launch_cells_c128(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st);
+cudaError_t launch_cells_c64(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st);
 cudaError_t launch_rows_f32(const OpDesc& d, int dtype, const StencilArgs& sa, int nbatch, cudaStream_t st);
 // The cp.async star / general kernel for an apply.
 cudaError_t launch_apply_cpasync(const OpDesc& d, int dtype, const StencilArgs& a, int nbatch, cudaStream_t st);

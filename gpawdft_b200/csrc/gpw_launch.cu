@@ -80,37 +80,15 @@ static cudaError_t run_direct(const StencilArgs& a0, const OpDesc& d, int nbatch
                     star_coefs_typed<typename EltTraits<T>::S>(d.sc));
 }
 
-template <typename T, int R, int MODE, bool EPI>
-static cudaError_t run_star_epi(const StencilArgs& a0, const OpDesc& d, int nbatch, cudaStream_t st) {
-  using C = StarCfg<R, T>;
-  StencilArgs a = a0;
-  const GridView& v = a.vout;
-  dim3 grid((v.n[2] + C::TZ - 1) / C::TZ, (v.n[1] + C::TY - 1) / C::TY, 1);
-  choose_chunks(v.n[0], (int64_t)grid.x * grid.y * nbatch, 2 * R + 2, a.zchunk, a.nchunk);
-  grid.z = a.nchunk * nbatch;
-  a.nblk_seg = grid.x * grid.y * a.nchunk;
-  const size_t smem = (size_t)C::NSTAGE * C::PS * sizeof(T);
-  using S = typename EltTraits<T>::S;
-  void (*kern)(StencilArgs, StarCoefsT<S>);
-  if constexpr (sizeof(T) >= 16)
-    kern = star_stencil_kernel_2cta<T, R, MODE, EPI>;
-  else
-    kern = star_stencil_kernel<T, R, MODE, EPI>;
-  static std::once_flag once;
-  cudaError_t e = cudaSuccess;
-  std::call_once(once, [&] { e = smem_optin(kern, smem); });
-  if (e != cudaSuccess) return e;
-  kern<<<grid, dim3(C::TZ, C::NTY), smem, st>>>(a, star_coefs_typed<S>(d.sc));  // NT threads
-  return cudaGetLastError();
-}
-
 template <typename T, int R, int MODE>
 static cudaError_t run_star(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
   if (direct_ok(a.vin, nbatch, sizeof(T))) return run_direct<T, R, MODE>(a, d, nbatch, st);
-  if constexpr (MODE == MODE_APPLY) {
-    if (a.pot || a.aux) return run_star_epi<T, R, MODE, true>(a, d, nbatch, st);
+  if constexpr (EltTraits<T>::cpx) {
+    static_assert(MODE == MODE_APPLY, "complex grids: applies only");
+    return sizeof(T) == 16 ? launch_cells_c128(a, d, nbatch, st) : launch_cells_c64(a, d, nbatch, st);
+  } else {
+    return sizeof(T) == 8 ? launch_cells_f64(MODE, a, d, nbatch, st) : launch_cells_f32(MODE, a, d, nbatch, st);
   }
-  return run_star_epi<T, R, MODE, false>(a, d, nbatch, st);
 }
 
 // Tile of a general-offset launch for element size es and radius mp: the
@@ -280,7 +258,8 @@ int stencil_blocks_per_member(const OpDesc& d, int mode, const GridView& v, int 
     int zc;
     const dim3 g = direct_grid(v, nbatch, zc);
     nblk = direct_ok(v, nbatch, 4) ? (int)(g.x * g.y) : 0;
-    nblk = std::max(nblk, blocks(32, d.real ? GPW_STAR_TY : GPW_STAR_TY / 2, 2 * d.R + 2));  // complex128: half-height tiles
+    // cell-staged tiles: at least 32 points wide and 20 rows high
+    nblk = std::max(nblk, (v.n[2] + 31) / 32 * ((v.n[1] + 19) / 20) * std::max(1, v.n[0] / (2 * d.R + 2)));
   } else {
     // the tile depends on the element size: the most CTAs over the op's types
     nblk = 0;

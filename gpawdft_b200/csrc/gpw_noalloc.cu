@@ -24,6 +24,7 @@
 #include <string>
 
 #include "gpw_internal.h"
+#include "gpw_star_cells.cuh"
 #include "gpw_stencil.cuh"
 
 namespace gpw {
@@ -79,20 +80,22 @@ void noalloc_chunks(int n0, int64_t tiles, int minz, int& zchunk, int& nchunk) {
 template <typename T, int R>
 cudaError_t star_residual(StencilArgs a, const OpDesc& d, int nbatch, bool launch, int64_t& nblk,
                           cudaStream_t st) {
-  using C = StarCfg<R, T>;
-  dim3 grid((a.vout.n[2] + C::TZ - 1) / C::TZ, (a.vout.n[1] + C::TY - 1) / C::TY, 1);
-  noalloc_chunks(a.vout.n[0], (int64_t)grid.x * grid.y * nbatch, 2 * R + 2, a.zchunk, a.nchunk);
-  grid.z = a.nchunk * nbatch;
+  // 32-wide tiles whatever the grid, at least 32 rows high; the limit counts
+  // (and the chunks are chosen for) tiles of 32 x 32 points
+  using C = CellsCfg<T, R, MODE_RESIDUAL, 32, (int)sizeof(T)>;
+  static_assert(C::TY >= 32, "no more blocks than the limit counts");
+  const int64_t tiles = (int64_t)((a.vout.n[2] + 31) / 32) * ((a.vout.n[1] + 31) / 32);
+  noalloc_chunks(a.vout.n[0], tiles * nbatch, 2 * R + 2, a.zchunk, a.nchunk);
+  nblk = tiles * a.nchunk;
+  const dim3 grid((a.vout.n[2] + C::TZ - 1) / C::TZ, (a.vout.n[1] + C::TY - 1) / C::TY, a.nchunk * nbatch);
   a.nblk_seg = grid.x * grid.y * a.nchunk;
-  nblk = a.nblk_seg;
   if (!launch) return cudaSuccess;
-  const size_t smem = (size_t)C::NSTAGE * C::PS * sizeof(T);
-  auto kern = star_stencil_kernel<T, R, MODE_RESIDUAL>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kern = star_cells_kernel<T, R, MODE_RESIDUAL, 32, (int)sizeof(T), 0, false>;
+  if (C::smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<grid, dim3(C::TZ, C::NTY), smem, st>>>(a, star_coefs_typed<typename EltTraits<T>::S>(d.sc));
+  kern<<<grid, dim3(C::NT), C::smem, st>>>(a, star_coefs_typed<typename EltTraits<T>::S>(d.sc));
   return cudaGetLastError();
 }
 

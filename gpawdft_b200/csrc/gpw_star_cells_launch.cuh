@@ -1,0 +1,101 @@
+// Launch of the cell-staged star stencil (gpw_star_cells.cuh): tile width,
+// cell size and axis-0 chunking.  Included by gpw_cells_f64.cu,
+// gpw_cells_f32.cu and gpw_cells_cpx.cu, which compile the element types in
+// parallel.
+#pragma once
+#include <algorithm>
+#include <mutex>
+
+#include "gpw_internal.h"
+#include "gpw_star_cells.cuh"
+#include "gpw_tma_launch.cuh"
+
+namespace gpw {
+
+// Rows of 16-byte cells: every row of the input, and the wrap of a periodic
+// row, on a 16-byte boundary.
+inline bool cells16_ok(const StencilArgs& a, size_t es, int nbatch) {
+  const GridView& v = a.vin;
+  return (reinterpret_cast<uintptr_t>(a.in) & 15u) == 0 && (v.n[2] * es) % 16 == 0 && (v.s1 * (int64_t)es) % 16 == 0 &&
+         (v.s0 * (int64_t)es) % 16 == 0 && (nbatch == 1 || (v.sb * (int64_t)es) % 16 == 0);
+}
+
+template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM>
+cudaError_t cells_run(StencilArgs a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  using C = CellsCfg<T, R, MODE, TZ, CELLB>;
+  auto kern = star_cells_kernel<T, R, MODE, TZ, CELLB, EPI, SYM>;
+  static std::once_flag once;
+  static cudaError_t oe = cudaSuccess;
+  static int per_sm = 1;
+  std::call_once(once, [&] {
+    oe = smem_optin_bytes(kern, C::smem);
+    if (oe == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::NT, C::smem) != cudaSuccess)
+      per_sm = 1;
+  });
+  if (oe != cudaSuccess) return oe;
+  const GridView& v = a.vout;
+  dim3 grid((v.n[2] + C::TZ - 1) / C::TZ, (v.n[1] + C::TY - 1) / C::TY, 1);
+  a.nchunk = tma_model_chunks(v.n[0], (int64_t)grid.x * grid.y * nbatch, R, (int64_t)std::max(1, per_sm) * num_sms());
+  grid.z = a.nchunk * nbatch;
+  a.nblk_seg = grid.x * grid.y * a.nchunk;
+  return launch_pdl(kern, grid, dim3(C::NT), C::smem, st, a, star_coefs_typed<typename EltTraits<T>::S>(d.sc));
+}
+
+template <typename T, int R, int MODE, int TZ, int CELLB, bool SYM>
+cudaError_t cells_term(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  if constexpr (MODE == MODE_APPLY) {
+    if (a.aux) return cells_run<T, R, MODE, TZ, CELLB, 2, SYM>(a, d, nbatch, st);
+    if (a.pot) return cells_run<T, R, MODE, TZ, CELLB, 1, SYM>(a, d, nbatch, st);
+  }
+  return cells_run<T, R, MODE, TZ, CELLB, 0, SYM>(a, d, nbatch, st);
+}
+
+template <typename T, int R, int MODE, int TZ>
+cudaError_t cells_form(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  constexpr int ES = (int)sizeof(T);
+  if (ES < 16 && cells16_ok(a, ES, nbatch)) return cells_term<T, R, MODE, TZ, 16, true>(a, d, nbatch, st);
+  return cells_term<T, R, MODE, TZ, ES, true>(a, d, nbatch, st);
+}
+
+// Tile widths: the one of the two whose tiles stage fewer cells for the grid
+// (radius 1 and 3, the stencils of GPAW's levels; one width for the others).
+template <typename T, int R, int MODE>
+cudaError_t cells_width(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  constexpr int TA = sizeof(T) == 4 ? 64 : 32, TB = sizeof(T) == 16 ? 24 : 48;
+  // other stencils than Laplacians: one width and cell size
+  if (!star_symmetric(d.sc, R)) return cells_term<T, R, MODE, TA, (int)sizeof(T), false>(a, d, nbatch, st);
+  if constexpr (R == 1 || R == 3) {
+    using CA = CellsCfg<T, R, MODE, TA, (int)sizeof(T)>;
+    using CB = CellsCfg<T, R, MODE, TB, (int)sizeof(T)>;
+    auto cells = [&](int tz, int ty, int box) {
+      return (int64_t)((a.vout.n[2] + tz - 1) / tz) * ((a.vout.n[1] + ty - 1) / ty) * box;
+    };
+    if (cells(TB, CB::TY, CB::H * CB::W) < cells(TA, CA::TY, CA::H * CA::W))
+      return cells_form<T, R, MODE, TB>(a, d, nbatch, st);
+  }
+  return cells_form<T, R, MODE, TA>(a, d, nbatch, st);
+}
+
+template <typename T, int MODE>
+cudaError_t cells_radius(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  switch (d.R) {
+    case 1: return cells_width<T, 1, MODE>(a, d, nbatch, st);
+    case 2: return cells_width<T, 2, MODE>(a, d, nbatch, st);
+    case 3: return cells_width<T, 3, MODE>(a, d, nbatch, st);
+    case 4: return cells_width<T, 4, MODE>(a, d, nbatch, st);
+  }
+  return cudaErrorInvalidValue;
+}
+
+template <typename T>
+cudaError_t cells_real(int mode, const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  switch (mode) {
+    case MODE_APPLY: return cells_radius<T, MODE_APPLY>(a, d, nbatch, st);
+    case MODE_RESIDUAL: return cells_radius<T, MODE_RESIDUAL>(a, d, nbatch, st);
+    case MODE_JACOBI: return cells_radius<T, MODE_JACOBI>(a, d, nbatch, st);
+  }
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace gpw

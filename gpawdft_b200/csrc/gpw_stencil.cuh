@@ -9,19 +9,15 @@
 // boundaries, wrapped addresses plus a phase fix-up for periodic ones) and
 // the halo is produced on the fly.
 //
-// Two kernels:
+// Kernels:
 //  * general_stencil_kernel -- any offsets within [-mp, mp]^3 (GUC Laplacians
 //    with diagonal directions, Mehrstellen, gradients of skew cells).  A ring
 //    of 2mp+2 planes lives in shared memory; every output gathers its
 //    coefficients in the reference's order with unfused multiply / add, so
 //    float64 results are bit-identical to c/bmgs/fd.c.
-//  * star_stencil_kernel -- star (cfd) stencils of radius R: register-blocked
-//    march along axis 0.  Each arriving plane contributes its in-plane part
-//    (axes 1, 2 from shared memory, PY rows per thread held in registers) and
-//    its axis-0 terms to 2R+1 running accumulators; an output plane is
-//    complete R planes after its centre arrives.  Fused multiply-adds; float64
-//    results agree with the reference to ~1e-16 relative.
-// Both support three epilogues: APPLY (out = A in), RESIDUAL (out = A in -
+//  * star (cfd) stencils: gpw_star_cells.cuh and, by shape, gpw_direct.cuh,
+//    gpw_rows.cuh, gpw_star_tma.cuh and gpw_bloch_tma.cuh.
+// All support three epilogues: APPLY (out = A in), RESIDUAL (out = A in -
 // rho and a deterministic sum of |out|^2) and JACOBI (one weighted-Jacobi
 // sweep, out = (1-w) in + w (rho - sum_{p!=0} c_p in[x+o_p]) / c_0).
 #pragma once
@@ -697,31 +693,6 @@ __global__ void __launch_bounds__(MehrCfg::NT, 2) mehrstellen_kernel(const Stenc
 }
 
 // ------------------------------------------------------------------ star
-// Tile TZ (axis 2) x TY (axis 1); PY consecutive axis-1 rows per thread.
-#ifndef GPW_STAR_TY
-#define GPW_STAR_TY 32
-#endif
-#ifndef GPW_STAR_PY
-#define GPW_STAR_PY 4
-#endif
-#ifndef GPW_STAR_NS
-#define GPW_STAR_NS 3
-#endif
-// 16-byte elements (complex128) take half-height tiles: two CTAs of 256
-// threads per SM (star_stencil_kernel_2cta) instead of one of 512, so one
-// CTA's plane barrier overlaps the other's work.
-template <int R, typename T>
-struct StarCfg {
-  static constexpr int TZ = 32;
-  static constexpr int PY = (sizeof(T) >= 16) ? (GPW_STAR_PY > 2 ? 2 : GPW_STAR_PY) : GPW_STAR_PY;
-  static constexpr int TY = (sizeof(T) >= 16) ? GPW_STAR_TY / 2 : GPW_STAR_TY;
-  static constexpr int NTY = TY / PY;
-  static constexpr int NT = TZ * NTY;
-  static constexpr int H = TY + 2 * R, W = TZ + 2 * R, PS = H * W;
-  static constexpr int NLD = (PS + NT - 1) / NT;  // plane cells loaded per thread
-  static constexpr int NSTAGE = GPW_STAR_NS;
-};
-
 struct StarCoefs {
   double cx[13], cy[13], cz[13];  // per-axis coefficients indexed offset + R (centres zero)
   double cc;                      // total centre (diagonal) coefficient
@@ -745,239 +716,6 @@ inline StarCoefsT<S> star_coefs_typed(const StarCoefs& sc) {
   }
   t.cc = (S)sc.cc;
   return t;
-}
-
-// Per-thread plane-load descriptors: the tile position in (axis 1, axis 2) is
-// fixed for the CTA, so each cell's in-plane source offset, validity and
-// wrap sides are computed once; a plane load is then one cp.async per cell.
-template <typename T, int R>
-struct StarLoader {
-  using C = StarCfg<R, T>;
-  int off[C::NLD];      // j1 * s1 + j2 (element offset inside a plane)
-  unsigned valid = 0;   // bit k: cell k is inside the grid or a periodic image
-  unsigned wrapped = 0; // bit k: cell k is a periodic image along axis 1 or 2
-  unsigned char side[C::NLD];  // wrap sides: bits 0-1 axis 1 (+1), bits 2-3 axis 2 (+1)
-
-  __device__ __forceinline__ void init(const GridView& v, const Boundary& bc, int y0, int x0) {
-    const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-#pragma unroll
-    for (int k = 0; k < C::NLD; ++k) {
-      const int idx = tid + k * C::NT;
-      const int r = idx / C::W, c = idx - r * C::W;
-      int j1 = 0, j2 = 0, s1 = -1, s2 = -1;
-      const bool ok = idx < C::PS && wrap_axis(y0 - R + r, v.n[1], bc.periodic[1], j1, s1) &&
-                      wrap_axis(x0 - R + c, v.n[2], bc.periodic[2], j2, s2);
-      off[k] = ok ? (int)((int64_t)j1 * v.s1 + j2) : 0;
-      if (ok) valid |= 1u << k;
-      if (ok && (s1 >= 0 || s2 >= 0)) wrapped |= 1u << k;
-      side[k] = (unsigned char)((s1 + 1) | ((s2 + 1) << 2));
-    }
-  }
-
-  __device__ __forceinline__ void load(T* slot, const T* in, const GridView& v, const Boundary& bc, int p) const {
-    const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    int j0, s0;
-    const bool ok0 = wrap_axis(p, v.n[0], bc.periodic[0], j0, s0);
-    const T* base = in + (int64_t)j0 * v.s0;
-#pragma unroll
-    for (int k = 0; k < C::NLD; ++k) {
-      const int idx = tid + k * C::NT;
-      if (C::PS % C::NT == 0 || idx < C::PS) {
-        const bool ok = ok0 && ((valid >> k) & 1u);
-        cp_async<sizeof(T)>(slot + idx, ok ? base + off[k] : in, ok);
-      }
-    }
-  }
-
-  // Bloch phases of the periodic images, axis by axis as the reference's
-  // chained halo copies apply them (each thread fixes its own copies).
-  __device__ __forceinline__ void fix(T* slot, const GridView& v, const Boundary& bc, int p) const {
-    if constexpr (EltTraits<T>::cpx) {
-      const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-      int j0, s0;
-      if (!wrap_axis(p, v.n[0], bc.periodic[0], j0, s0)) return;
-      // on a plane inside the grid only the in-plane periodic images change
-      const unsigned todo = s0 < 0 ? wrapped : valid;
-      if (!todo) return;
-#pragma unroll
-      for (int k = 0; k < C::NLD; ++k) {
-        const int idx = tid + k * C::NT;
-        if (idx >= C::PS || !((todo >> k) & 1u)) continue;
-        const int s1 = (side[k] & 3) - 1, s2 = ((side[k] >> 2) & 3) - 1;
-        T val = slot[idx];
-        if (s0 >= 0) val = phase_mul(bc.ph[0][s0], val);
-        if (s1 >= 0) val = phase_mul(bc.ph[1][s1], val);
-        if (s2 >= 0) val = phase_mul(bc.ph[2][s2], val);
-        slot[idx] = val;
-      }
-    }
-  }
-};
-
-// EPI: an apply with a potential or aux term (a.pot / a.aux); the plain
-// apply is compiled without their loads and branches.
-template <typename T, int R, int MODE, bool EPI>
-__device__ __forceinline__ void star_stencil_body(const StencilArgs& a, const StarCoefsT<typename EltTraits<T>::S>& k) {
-  using C = StarCfg<R, T>;
-  using S = typename EltTraits<T>::S;
-  constexpr int PY = C::PY, W = C::W, PS = C::PS, NS = C::NSTAGE;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* ring = reinterpret_cast<T*>(smem_raw);
-  __shared__ double red[32];
-
-  const int b = blockIdx.z / a.nchunk, chunk = blockIdx.z - b * a.nchunk;
-  if (a.active && !a.active[b]) return;
-  const int x0 = blockIdx.x * C::TZ, y0 = blockIdx.y * C::TY;
-  const int n0 = a.vout.n[0];
-  const int z0 = chunk * a.zchunk;
-  const int z1 = min(n0, z0 + a.zchunk);
-  const T* in = static_cast<const T*>(a.in) + (int64_t)b * a.vin.sb;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int x = x0 + tx;
-  const int yb = ty * PY;  // first local row of this thread
-  const bool xin = x < a.vout.n[2];
-  double sumsq = 0.0;
-
-  StarLoader<T, R> ld;
-  ld.init(a.vin, a.bc, y0, x0);
-
-  T acc[PY][2 * R + 1];
-  T cur[PY][R + 1];  // JACOBI: centre values of the last R+1 planes
-#pragma unroll
-  for (int j = 0; j < PY; ++j) {
-#pragma unroll
-    for (int m = 0; m < 2 * R + 1; ++m) acc[j][m] = zero<T>();
-#pragma unroll
-    for (int m = 0; m < R + 1; ++m) cur[j][m] = zero<T>();
-  }
-
-  if (z0 < z1) {
-    const int pfirst = z0 - R, plast = z1 - 1 + R;
-    const int nsteps = plast - pfirst + 1;
-#pragma unroll
-    for (int st = 0; st < NS - 1; ++st) {
-      if (st < nsteps) ld.load(ring + st * PS, in, a.vin, a.bc, pfirst + st);
-      cp_async_commit();
-    }
-    for (int s = 0; s < nsteps; ++s) {
-      const int p = pfirst + s;
-      {
-        const int sn = s + NS - 1;
-        if (sn < nsteps) ld.load(ring + (sn % NS) * PS, in, a.vin, a.bc, pfirst + sn);
-        cp_async_commit();
-      }
-      // prefetch rho for the output plane that completes at this step
-      const int o = p - R;
-      T rho[PY];
-      if constexpr (MODE != MODE_APPLY) {
-#pragma unroll
-        for (int j = 0; j < PY; ++j) {
-          const int y = y0 + yb + j;
-          rho[j] = zero<T>();
-          if (o >= z0 && xin && y < a.vout.n[1])
-            rho[j] = static_cast<const T*>(a.rho)[(int64_t)b * a.vrho.sb + (int64_t)o * a.vrho.s0 +
-                                                  (int64_t)y * a.vrho.s1 + x];
-        }
-      }
-      cp_async_wait<NS - 1>();
-      T* sl = ring + (s % NS) * PS;
-      if (EltTraits<T>::cpx && a.bc.use_phase) ld.fix(sl, a.vin, a.bc, p);
-      __syncthreads();
-
-      // column of PY + 2R values along axis 1 at this thread's x
-      T col[PY + 2 * R];
-#pragma unroll
-      for (int i = 0; i < PY + 2 * R; ++i) col[i] = sl[(yb + i) * W + tx + R];
-#pragma unroll
-      for (int j = 0; j < PY; ++j) {
-        const T v = col[j + R];
-        // in-plane part: centre + axis-1 + axis-2 neighbours (coefficients
-        // are read from the kernel-parameter bank)
-        T part = scale((MODE == MODE_JACOBI) ? S(0) : (S)k.cc, v);
-#pragma unroll
-        for (int q = 1; q <= R; ++q) {
-          part = fmac((S)k.cy[R + q], col[j + R + q], part);
-          part = fmac((S)k.cy[R - q], col[j + R - q], part);
-        }
-        const T* row = sl + (yb + j + R) * W + tx + R;
-#pragma unroll
-        for (int q = 1; q <= R; ++q) {
-          part = fmac((S)k.cz[R + q], row[q], part);
-          part = fmac((S)k.cz[R - q], row[-q], part);
-        }
-        if constexpr (MODE == MODE_APPLY && EPI) {
-          // local potential of this (in-range) plane: its part is output p's
-          const int y = y0 + yb + j;
-          if (a.pot && p >= z0 && p < z1 && xin && y < a.vout.n[1])
-            part = fmac(static_cast<const S*>(a.pot)[(int64_t)p * a.vout.s0 + (int64_t)y * a.vout.s1 + x], v, part);
-        }
-        // scatter along axis 0: output plane p-R+m receives offset R-m
-#pragma unroll
-        for (int m = 0; m < 2 * R + 1; ++m) {
-          if (m == R)
-            acc[j][m] = add(acc[j][m], part);
-          else
-            acc[j][m] = fmac((S)k.cx[2 * R - m], v, acc[j][m]);
-        }
-        if constexpr (MODE == MODE_JACOBI) {
-#pragma unroll
-          for (int m = 0; m < R; ++m) cur[j][m] = cur[j][m + 1];
-          cur[j][R] = v;
-        }
-      }
-      // output plane o = p - R is complete
-      if (o >= z0) {
-#pragma unroll
-        for (int j = 0; j < PY; ++j) {
-          const int y = y0 + yb + j;
-          if (xin && y < a.vout.n[1]) {
-            const int64_t oi = (int64_t)b * a.vout.sb + (int64_t)o * a.vout.s0 + (int64_t)y * a.vout.s1 + x;
-            const T av = acc[j][0];
-            if constexpr (MODE == MODE_APPLY) {
-              static_cast<T*>(a.out)[oi] =
-                  (EPI && a.aux) ? fmac((S)a.aux_scale, static_cast<const T*>(a.aux)[oi], av) : av;
-            } else if constexpr (MODE == MODE_RESIDUAL) {
-              const T r = sub(av, rho[j]);
-              if (a.out) static_cast<T*>(a.out)[oi] = r;
-              sumsq += norm2(r);
-            } else {
-              if constexpr (!EltTraits<T>::cpx) {
-                const S w = (S)a.w;
-                const S wc = w / (S)a.c0;
-                static_cast<T*>(a.out)[oi] = (S(1) - w) * cur[j][0] + wc * (rho[j] - av);
-              }
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < PY; ++j) {
-#pragma unroll
-        for (int m = 0; m < 2 * R; ++m) acc[j][m] = acc[j][m + 1];
-        acc[j][2 * R] = zero<T>();
-      }
-      __syncthreads();
-    }
-  }
-  if constexpr (MODE == MODE_RESIDUAL) {
-    if (!a.gsum.partial) return;  // residual without its norm
-    double tot = block_sum(sumsq, red);
-    const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * chunk);
-    grid_sum_finish(a.gsum, b, blk, a.nblk_seg, tot, red);
-  }
-}
-
-template <typename T, int R, int MODE, bool EPI = false>
-__global__ void __launch_bounds__(StarCfg<R, T>::NT)
-    star_stencil_kernel(const StencilArgs a, const StarCoefsT<typename EltTraits<T>::S> k) {
-  star_stencil_body<T, R, MODE, EPI>(a, k);
-}
-
-// 16-byte elements: the same kernel with registers capped for two CTAs per SM
-template <typename T, int R, int MODE, bool EPI = false>
-__global__ void __launch_bounds__(StarCfg<R, T>::NT, 2)
-    star_stencil_kernel_2cta(const StencilArgs a, const StarCoefsT<typename EltTraits<T>::S> k) {
-  star_stencil_body<T, R, MODE, EPI>(a, k);
 }
 
 }  // namespace gpw
