@@ -166,7 +166,12 @@ static cudaError_t run_general(const StencilArgs& a0, const OpDesc& d, int nbatc
   general_tile(mp, sizeof(T), tz, ty, blocked);
   if (blocked && (tz != GenBlk<T, 1>::TZ || ty != GenBlk<T, 1>::TY)) return cudaErrorInvalidConfiguration;
   dim3 grid((v.n[2] + tz - 1) / tz, (v.n[1] + ty - 1) / ty, 1);
+  // (chunks for whole waves of two CTAs per SM, each chunk paying 2mp planes
+  // again; the norm's partial slots count the chunks choose_chunks gives)
   choose_chunks(v.n[0], (int64_t)grid.x * grid.y * nbatch, 2 * mp + 2, a.zchunk, a.nchunk);
+  const int nc = wave_chunks(v.n[0], (int64_t)grid.x * grid.y * nbatch, 2 * mp, 2LL * num_sms(), a.nchunk);
+  a.zchunk = (v.n[0] + nc - 1) / nc;
+  a.nchunk = (v.n[0] + a.zchunk - 1) / a.zchunk;
   grid.z = a.nchunk * nbatch;
   a.nblk_seg = grid.x * grid.y * a.nchunk;
   // planes loaded ahead: as many (up to 4) as keep two CTAs per SM

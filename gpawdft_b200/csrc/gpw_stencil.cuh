@@ -400,8 +400,8 @@ __global__ void __launch_bounds__(GenBlk<T, MP, PY_, NTY_>::NT, 2)
       }
     };
     // one commit group for the first 2mp + 1 planes, then one per plane: at
-    // output plane o the groups of planes o + mp + 1 .. o + mp + D may still
-    // be in flight
+    // output plane o the groups of planes o + mp + 1 .. o + mp + D - 1 may
+    // still be in flight
     for (int p = z0 - MP; p <= z0 + MP; ++p) load(p);
     cp_async_commit();
     for (int d = 1; d < D; ++d) {
@@ -425,13 +425,11 @@ __global__ void __launch_bounds__(GenBlk<T, MP, PY_, NTY_>::NT, 2)
         rbase[i][j] = (int64_t)b * a.vrho.sb + (int64_t)y * a.vrho.s1 + x;
       }
     for (int o = z0; o < z1; ++o) {
-      if (o + D < z1) load(o + MP + D);
-      cp_async_commit();
       switch (D) {
-        case 1: cp_async_wait<1>(); break;
-        case 2: cp_async_wait<2>(); break;
-        case 3: cp_async_wait<3>(); break;
-        default: cp_async_wait<4>(); break;
+        case 1: cp_async_wait<0>(); break;
+        case 2: cp_async_wait<1>(); break;
+        case 3: cp_async_wait<2>(); break;
+        default: cp_async_wait<3>(); break;
       }
       if (bc.use_phase) {
         if (o == z0) {
@@ -441,6 +439,9 @@ __global__ void __launch_bounds__(GenBlk<T, MP, PY_, NTY_>::NT, 2)
         }
       }
       __syncthreads();
+      // the slot refilled held plane o - MP - 1, last read before this barrier
+      if (o + D < z1) load(o + MP + D);
+      cp_async_commit();
       const int cs = (o - z0 + MP) % NP;  // slot of plane o
       const GenTab<S>* tc = tab + cs * ncoef;
       const unsigned char* co = cen + cs * PS * (int)sizeof(T);
@@ -493,7 +494,6 @@ __global__ void __launch_bounds__(GenBlk<T, MP, PY_, NTY_>::NT, 2)
           }
         }
       }
-      __syncthreads();
     }
   }
   if constexpr (MODE == MODE_RESIDUAL) {
@@ -608,15 +608,16 @@ __global__ void __launch_bounds__(MehrCfg::NT, 2) mehrstellen_kernel(const Stenc
     // this thread's first output cell (row 2 ty + 1, column 2 tx + 1 of a slot)
     const int cell = (2 * ty + 1) * W + 2 * tx + 1;
     for (int o = z0; o < z1; ++o) {
-      if (o + D < z1) load(o + 1 + D);
-      cp_async_commit();
       switch (D) {
-        case 1: cp_async_wait<1>(); break;
-        case 2: cp_async_wait<2>(); break;
-        case 3: cp_async_wait<3>(); break;
-        default: cp_async_wait<4>(); break;
+        case 1: cp_async_wait<0>(); break;
+        case 2: cp_async_wait<1>(); break;
+        case 3: cp_async_wait<2>(); break;
+        default: cp_async_wait<3>(); break;
       }
       __syncthreads();
+      // the slot refilled held plane o - 2, last read before this barrier
+      if (o + D < z1) load(o + 1 + D);
+      cp_async_commit();
       const int cs = (o - z0 + 1) % NP;
       const T* pm = ring + ((cs + NP - 1) % NP) * PS + cell;  // plane o - 1
       const T* pc = ring + cs * PS + cell;                    // plane o
@@ -681,7 +682,6 @@ __global__ void __launch_bounds__(MehrCfg::NT, 2) mehrstellen_kernel(const Stenc
           }
         }
       }
-      __syncthreads();
     }
   }
   if constexpr (MODE == MODE_RESIDUAL) {
