@@ -42,6 +42,7 @@ struct CoarseLevel {
   double cm[3], cp[3];    // neighbour coefficients at offsets -1 / +1 per axis
   int npre, npost;
   double w[CG_MAXW];      // pre-sweep weights, then post-sweep weights
+  double wc[CG_MAXW];     // w / cc, divided in the kernel's element type
 };
 
 struct CoarseArgs {
@@ -142,11 +143,12 @@ __device__ __forceinline__ void pg_points(const PadGeom& g, F body) {
   }
 }
 
+// sweep s (index into the level's weights) from src to dst
 template <bool PER, typename S>
 __device__ __forceinline__ void pg_jacobi(const CoarseLevel& L, const S* __restrict__ src, S* __restrict__ dst,
-                                          const S* __restrict__ rho, double wd) {
+                                          const S* __restrict__ rho, int s) {
   const PadGeom g(L);
-  const S w = (S)wd, wc = w / (S)L.cc;
+  const S w = (S)L.w[s], wc = (S)L.wc[s];
   const S c0m = (S)L.cm[0], c0p = (S)L.cp[0], c1m = (S)L.cm[1], c1p = (S)L.cp[1], c2m = (S)L.cm[2],
           c2p = (S)L.cp[2];
   pg_points(g, [&](int i0, int i1, int i2, int k) {
@@ -161,28 +163,28 @@ __device__ __forceinline__ void pg_jacobi(const CoarseLevel& L, const S* __restr
   __syncthreads();
 }
 
-// n sweeps on the buffers P, starting from P[c]; returns the buffer of the
-// result.  On levels of at most PG_U points a thread each thread finds its
-// points (index divisions, boundaries) once for all sweeps, whose passes are
-// then as short as their barrier: a sweep of a 10^3 or 7^3 level otherwise
-// spends most of its ~1 us on indices.
+// Sweeps s0 .. s0 + n - 1 on the buffers P, starting from P[c]; returns the
+// buffer of the result.  On levels of at most PG_U points a thread each thread
+// finds its points once for all sweeps, and on periodic ones its neighbours'
+// wrapped positions too, so that only the last sweep writes halo images.
 constexpr int PG_U = 8;
 template <bool PER, typename S>
 __device__ __forceinline__ int pg_sweeps(const CoarseLevel& L, S* const (&P)[2], int c, const S* __restrict__ rho,
-                                         const double* w, int n) {
+                                         int s0, int n) {
   const PadGeom g(L);
   const int ncol = g.n1 * g.n2, pts = ncol * g.n0, nt = blockDim.x;
-  if (n < 2 || ncol >= nt || pts > PG_U * nt) {
-    for (int s = 0; s < n; ++s, c = 1 - c) pg_jacobi<PER>(L, P[c], P[1 - c], rho, w[s]);
+  constexpr int U = PER ? PG_U / 2 : PG_U;
+  if (n < 2 || ncol >= nt || pts > U * nt) {
+    for (int s = 0; s < n; ++s, c = 1 - c) pg_jacobi<PER>(L, P[c], P[1 - c], rho, s0 + s);
     return c;
   }
   const S c0m = (S)L.cm[0], c0p = (S)L.cp[0], c1m = (S)L.cm[1], c1p = (S)L.cp[1], c2m = (S)L.cm[2],
           c2p = (S)L.cp[2];
-  int k[PG_U];
-  unsigned m[PG_U];
-  S r[PG_U];
+  int k[U];
+  unsigned m[U];
+  S r[U];
 #pragma unroll
-  for (int u = 0; u < PG_U; ++u) {
+  for (int u = 0; u < U; ++u) {
     const int i = threadIdx.x + u * nt;
     k[u] = -1;
     m[u] = 0;
@@ -198,21 +200,25 @@ __device__ __forceinline__ int pg_sweeps(const CoarseLevel& L, S* const (&P)[2],
   for (int s = 0; s < n; ++s, c = 1 - c) {
     const S* src = P[c];
     S* dst = P[1 - c];
-    const S ws = (S)w[s], wc = ws / (S)L.cc;
+    const S ws = (S)L.w[s0 + s], wc = (S)L.wc[s0 + s];
 #pragma unroll
-    for (int u = 0; u < PG_U; ++u) {
+    for (int u = 0; u < U; ++u) {
       if (u * nt >= pts) break;
       if (k[u] < 0) continue;
       const int q = k[u];
-      S av = c2m * src[q - 1];
-      av = fmac(c2p, src[q + 1], av);
-      av = fmac(c1m, src[q - g.sy], av);
-      av = fmac(c1p, src[q + g.sy], av);
-      av = fmac(c0m, src[q - g.sz], av);
-      av = fmac(c0p, src[q + g.sz], av);
+      // the neighbours: the other end of a periodic axis (m = 0: none)
+      const int b2 = PER && (m[u] & 16u) ? g.n2 - 1 : -1, a2 = PER && (m[u] & 32u) ? 1 - g.n2 : 1;
+      const int b1 = (PER && (m[u] & 4u) ? g.n1 - 1 : -1) * g.sy, a1 = (PER && (m[u] & 8u) ? 1 - g.n1 : 1) * g.sy;
+      const int b0 = (PER && (m[u] & 1u) ? g.n0 - 1 : -1) * g.sz, a0 = (PER && (m[u] & 2u) ? 1 - g.n0 : 1) * g.sz;
+      S av = c2m * src[q + b2];
+      av = fmac(c2p, src[q + a2], av);
+      av = fmac(c1m, src[q + b1], av);
+      av = fmac(c1p, src[q + a1], av);
+      av = fmac(c0m, src[q + b0], av);
+      av = fmac(c0p, src[q + a0], av);
       const S v = (S(1) - ws) * src[q] + wc * (r[u] - av);
       dst[q] = v;
-      if (PER && m[u]) g.images(dst, q, m[u], v);
+      if (PER && m[u] && s + 1 == n) g.images(dst, q, m[u], v);
     }
     __syncthreads();
   }
@@ -316,10 +322,10 @@ __device__ void coarse_vcycle_padded(const CoarseArgs& a, S* sm, int b) {
     const S* rho = sm + L.base + 2 * L.pts;
     int c = 0;
     if (l == nl - 1) {
-      cur[l] = pg_sweeps<PER>(L, P, c, rho, L.w + L.npre, L.npost);
+      cur[l] = pg_sweeps<PER>(L, P, c, rho, L.npre, L.npost);
       break;
     }
-    c = pg_sweeps<PER>(L, P, c, rho, L.w, L.npre);
+    c = pg_sweeps<PER>(L, P, c, rho, 0, L.npre);
     cur[l] = c;
     pg_residual<PER>(L, P[c], P[1 - c], rho);
     const CoarseLevel& C = a.lv[l + 1];
@@ -332,7 +338,7 @@ __device__ void coarse_vcycle_padded(const CoarseArgs& a, S* sm, int b) {
     const S* rho = sm + L.base + 2 * L.pts;
     int c = cur[l];
     pg_interp_sub<PER>(L, P[c], P[1 - c], C, sm + C.base + cur[l + 1] * C.pts);
-    cur[l] = pg_sweeps<PER>(L, P, 1 - c, rho, L.w + L.npre, L.npost);
+    cur[l] = pg_sweeps<PER>(L, P, 1 - c, rho, L.npre, L.npost);
   }
   {
     const CoarseLevel& L = a.lv[0];
@@ -547,7 +553,7 @@ __global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(c
   int c = 0;
   slab_exchange(cl, P[0], rank, np, npm, gs.sz);
   for (int s = t.first_done; s < T.npre; ++s, c = 1 - c) {
-    pg_jacobi<false>(Ls, P[c], P[1 - c], rho, T.w[s]);
+    pg_jacobi<false>(Ls, P[c], P[1 - c], rho, s);
     slab_exchange(cl, P[1 - c], rank, np, npm, gs.sz);
   }
   pg_residual<false>(Ls, P[c], P[1 - c], rho);
@@ -557,7 +563,7 @@ __global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(c
   int d = 0;
   slab_exchange(cl, Q[0], rank, mp, mpm, gu.sz);  // (zeros: keeps the barrier sequence uniform)
   for (int s = 0; s < U.npre; ++s, d = 1 - d) {
-    pg_jacobi<false>(Us, Q[d], Q[1 - d], rho2, U.w[s]);
+    pg_jacobi<false>(Us, Q[d], Q[1 - d], rho2, s);
     slab_exchange(cl, Q[1 - d], rank, mp, mpm, gu.sz);
   }
   pg_residual<false>(Us, Q[d], Q[1 - d], rho2);
@@ -588,7 +594,7 @@ __global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(c
   d = 1 - d;
   slab_exchange(cl, Q[d], rank, mp, mpm, gu.sz);
   for (int s = 0; s < U.npost; ++s, d = 1 - d) {
-    pg_jacobi<false>(Us, Q[d], Q[1 - d], rho2, U.w[U.npre + s]);
+    pg_jacobi<false>(Us, Q[d], Q[1 - d], rho2, U.npre + s);
     slab_exchange(cl, Q[1 - d], rank, mp, mpm, gu.sz);
   }
   // ---- top level: interpolation from the second level's slab (its halo planes included), post-sweeps
@@ -596,7 +602,7 @@ __global__ void __launch_bounds__(CG_CLUSTER_THREADS, 2) cluster_vcycle_kernel(c
   c = 1 - c;
   slab_exchange(cl, P[c], rank, np, npm, gs.sz);
   for (int s = 0; s < T.npost; ++s, c = 1 - c) {
-    pg_jacobi<false>(Ls, P[c], P[1 - c], rho, T.w[T.npre + s]);
+    pg_jacobi<false>(Ls, P[c], P[1 - c], rho, T.npre + s);
     if (s + 1 < T.npost) slab_exchange(cl, P[1 - c], rank, np, npm, gs.sz);
   }
   {

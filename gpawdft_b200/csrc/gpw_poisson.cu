@@ -458,6 +458,12 @@ const OpDesc* operator_desc(const gpw_operator* op);
 const TrDesc* transformer_desc(const gpw_transformer* tr);
 }  // namespace gpw
 
+// The sweeps' w / cc, divided in the element type (a division per sweep and
+// thread in the kernel was a good part of a small level's pass).
+static void sweep_lengths(CoarseLevel& c, bool f32) {
+  for (int i = 0; i < c.npre + c.npost; ++i) c.wc[i] = f32 ? (double)((float)c.w[i] / (float)c.cc) : c.w[i] / c.cc;
+}
+
 // Choose the first level of the coarse one-CTA kernel for form p (0 float64,
 // 1 float32) and fill its arguments: the deepest suffix of levels (never
 // level 0) that are real 7-point star Laplacians relaxed by Jacobi and whose
@@ -522,6 +528,7 @@ static void setup_cluster_top(gpw_poisson* ps, bool zero, size_t es) {
   c.npost = (int)L.wpost[1].size();
   for (int i = 0; i < c.npre; ++i) c.w[i] = L.wpre[1][i];
   for (int i = 0; i < c.npost; ++i) c.w[c.npre + i] = L.wpost[1][i];
+  sweep_lengths(c, true);
   t.L2 = U;
   t.slab_pts = (int)slab;
   t.slab2_pts = (int)slab2;
@@ -598,6 +605,7 @@ static void setup_coarse(gpw_poisson* ps, int p) {
     c.npost = (int)L.wpost[p].size();
     for (int i = 0; i < c.npre; ++i) c.w[i] = L.wpre[p][i];
     for (int i = 0; i < c.npost; ++i) c.w[c.npre + i] = L.wpost[p][i];
+    sweep_lengths(c, p == 1);
   }
   ps->lc[p] = lc;
   ps->csmem[p] = bytes;
