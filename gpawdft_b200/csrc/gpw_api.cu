@@ -147,11 +147,27 @@ int build_opdesc(OpDesc& d, const double* coefs, const int64_t* offsets, int nco
   R = std::max(R, 1);
   d.star = star && R <= 6;
   d.R = R;
-  std::memset(&d.sc, 0, sizeof(d.sc));
-  if (d.star) {
+  // a star and one diagonal of axes 0 and 1 (the Laplacian of a hexagonal
+  // cell whose third axis is perpendicular)
+  d.slope = 0;
+  if (!star && R <= 3) {
+    bool up = true, down = true;
     for (int p = 0; p < ncoef; ++p) {
       const int* o = &d.off[3 * p];
-      if (o[0] == 0 && o[1] == 0 && o[2] == 0)
+      const int nz = (o[0] != 0) + (o[1] != 0) + (o[2] != 0);
+      if (nz < 2) continue;
+      up = up && o[2] == 0 && o[1] == o[0];
+      down = down && o[2] == 0 && o[1] == -o[0];
+    }
+    d.slope = up ? 1 : (down ? -1 : 0);
+  }
+  std::memset(&d.sc, 0, sizeof(d.sc));
+  if (d.star || d.slope) {
+    for (int p = 0; p < ncoef; ++p) {
+      const int* o = &d.off[3 * p];
+      if (o[0] != 0 && o[1] != 0)
+        d.sc.cd[o[0] + R] += coefs[p];
+      else if (o[0] == 0 && o[1] == 0 && o[2] == 0)
         d.sc.cc += coefs[p];
       else if (o[0] != 0)
         d.sc.cx[o[0] + R] += coefs[p];
@@ -161,6 +177,13 @@ int build_opdesc(OpDesc& d, const double* coefs, const int64_t* offsets, int nco
         d.sc.cz[o[2] + R] += coefs[p];
     }
   }
+  // (a coefficient of 0 would spread infinities and NaN that the operator
+  // does not reach: all 8R + 1 points)
+  const double* lines[4] = {d.sc.cx, d.sc.cy, d.sc.cz, d.sc.cd};
+  for (int q = 1; q <= R && d.slope; ++q)
+    for (const double* c : lines)
+      if (c[R + q] == 0.0 || c[R + q] != c[R - q]) d.slope = 0;
+  if (d.sc.cc == 0.0) d.slope = 0;
   // Jacobi on the star kernel: coefs[0] must be the (unique) centre, which the
   // reference assumes (c/bmgs/relax.c sums c = 1 .. ncoefs-1 and divides by c_0)
   int ncentre = 0;

@@ -69,6 +69,7 @@ struct OpDesc {
   bool star;             // star kernel eligible for APPLY / RESIDUAL
   bool star_jacobi;      // star kernel eligible for JACOBI (centre first, unique)
   int R;                 // star radius
+  int slope;             // +-1: a star and one diagonal (q, slope q, 0) of axes 0 and 1, R <= 3, equal at +-q; else 0
   StarCoefs sc;
   GeneralCoefs gc;
   double diag;           // get_diagonal_element

@@ -90,7 +90,7 @@ cudaError_t star_residual(StencilArgs a, const OpDesc& d, int nbatch, bool launc
   const dim3 grid((a.vout.n[2] + C::TZ - 1) / C::TZ, (a.vout.n[1] + C::TY - 1) / C::TY, a.nchunk * nbatch);
   a.nblk_seg = grid.x * grid.y * a.nchunk;
   if (!launch) return cudaSuccess;
-  auto kern = star_cells_kernel<T, R, MODE_RESIDUAL, 32, (int)sizeof(T), 0, false>;
+  auto kern = star_cells_kernel<T, R, MODE_RESIDUAL, 32, (int)sizeof(T), 0, false, 0>;
   if (C::smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
     if (e != cudaSuccess) return e;

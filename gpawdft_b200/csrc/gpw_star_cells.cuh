@@ -55,7 +55,13 @@ struct CellsCfg {
 // SYM: the coefficients at +q and -q are equal on every axis (a Laplacian):
 // 3R + 1 coefficients stay in uniform registers, where 6R + 1 were loaded again
 // on every plane.
-template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM>
+// SLOPE: +-1 for a star and the diagonal (q, SLOPE q, 0) of axes 0 and 1,
+// whose terms scatter with the axis-0 ones from the column of rows a thread
+// holds anyway.  The centre, the largest term, comes after the in-plane
+// ones, so that fewer partial sums of its size are rounded (60^2 x 84 normal
+// values, R = 3: error against extended precision 1.3e-16; 1.8e-16 with the
+// centre first, 2.3e-16 for the general kernel's order).
+template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM, int SLOPE>
 __global__ void __launch_bounds__(CellsCfg<T, R, MODE, TZ, CELLB>::NT, (R <= 3 ? 2 : 1))
     star_cells_kernel(const StencilArgs a, const StarCoefsT<typename EltTraits<T>::S> k) {
   using C = CellsCfg<T, R, MODE, TZ, CELLB>;
@@ -262,7 +268,10 @@ __global__ void __launch_bounds__(CellsCfg<T, R, MODE, TZ, CELLB>::NT, (R <= 3 ?
               P part, pz;
 #pragma unroll
               for (int e = 0; e < VEC; e += 2) {
-                mul_pair((MODE == MODE_JACOBI) ? S(0) : k.cc, c.v[e], c.v[e + 1], part.v[e], part.v[e + 1]);
+                if constexpr (SLOPE != 0)
+                  part.v[e] = part.v[e + 1] = S(0);
+                else
+                  mul_pair((MODE == MODE_JACOBI) ? S(0) : k.cc, c.v[e], c.v[e + 1], part.v[e], part.v[e + 1]);
                 pz.v[e] = pz.v[e + 1] = S(0);
               }
 #pragma unroll
@@ -301,7 +310,10 @@ __global__ void __launch_bounds__(CellsCfg<T, R, MODE, TZ, CELLB>::NT, (R <= 3 ?
               }
               P& am = acc[j][R];
 #pragma unroll
-              for (int e = 0; e < VEC; e += 2) add_pair(part.v[e], part.v[e + 1], am.v[e], am.v[e + 1]);
+              for (int e = 0; e < VEC; e += 2) {
+                add_pair(part.v[e], part.v[e + 1], am.v[e], am.v[e + 1]);
+                if constexpr (SLOPE != 0) fma_pair(k.cc, c.v[e], c.v[e + 1], am.v[e], am.v[e + 1]);
+              }
             }
             // scatter along axis 0: output plane p-R+m receives offset R-m
 #pragma unroll
@@ -311,6 +323,12 @@ __global__ void __launch_bounds__(CellsCfg<T, R, MODE, TZ, CELLB>::NT, (R <= 3 ?
 #pragma unroll
                 for (int e = 0; e < VEC; e += 2)
                   fma_pair(k.cx[SYM && m > R ? m : 2 * R - m], c.v[e], c.v[e + 1], am.v[e], am.v[e + 1]);
+                if constexpr (SLOPE != 0) {
+                  const P& d = col[j + R + SLOPE * (R - m)];
+#pragma unroll
+                  for (int e = 0; e < VEC; e += 2)
+                    fma_pair(k.cd[SYM && m > R ? m : 2 * R - m], d.v[e], d.v[e + 1], am.v[e], am.v[e + 1]);
+                }
               }
           }
         }

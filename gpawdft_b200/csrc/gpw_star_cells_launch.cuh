@@ -20,10 +20,10 @@ inline bool cells16_ok(const StencilArgs& a, size_t es, int nbatch) {
          (v.s0 * (int64_t)es) % 16 == 0 && (nbatch == 1 || (v.sb * (int64_t)es) % 16 == 0);
 }
 
-template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM>
+template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM, int SLOPE>
 cudaError_t cells_run(StencilArgs a, const OpDesc& d, int nbatch, cudaStream_t st) {
   using C = CellsCfg<T, R, MODE, TZ, CELLB>;
-  auto kern = star_cells_kernel<T, R, MODE, TZ, CELLB, EPI, SYM>;
+  auto kern = star_cells_kernel<T, R, MODE, TZ, CELLB, EPI, SYM, SLOPE>;
   static std::once_flag once;
   static cudaError_t oe = cudaSuccess;
   static int per_sm = 1;
@@ -42,13 +42,13 @@ cudaError_t cells_run(StencilArgs a, const OpDesc& d, int nbatch, cudaStream_t s
   return launch_pdl(kern, grid, dim3(C::NT), C::smem, st, a, star_coefs_typed<typename EltTraits<T>::S>(d.sc));
 }
 
-template <typename T, int R, int MODE, int TZ, int CELLB, bool SYM>
+template <typename T, int R, int MODE, int TZ, int CELLB, bool SYM, int SLOPE = 0>
 cudaError_t cells_term(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
   if constexpr (MODE == MODE_APPLY) {
-    if (a.aux) return cells_run<T, R, MODE, TZ, CELLB, 2, SYM>(a, d, nbatch, st);
-    if (a.pot) return cells_run<T, R, MODE, TZ, CELLB, 1, SYM>(a, d, nbatch, st);
+    if (a.aux) return cells_run<T, R, MODE, TZ, CELLB, 2, SYM, SLOPE>(a, d, nbatch, st);
+    if (a.pot) return cells_run<T, R, MODE, TZ, CELLB, 1, SYM, SLOPE>(a, d, nbatch, st);
   }
-  return cells_run<T, R, MODE, TZ, CELLB, 0, SYM>(a, d, nbatch, st);
+  return cells_run<T, R, MODE, TZ, CELLB, 0, SYM, SLOPE>(a, d, nbatch, st);
 }
 
 template <typename T, int R, int MODE, int TZ>
@@ -56,6 +56,24 @@ cudaError_t cells_form(const StencilArgs& a, const OpDesc& d, int nbatch, cudaSt
   constexpr int ES = (int)sizeof(T);
   if (ES < 16 && cells16_ok(a, ES, nbatch)) return cells_term<T, R, MODE, TZ, 16, true>(a, d, nbatch, st);
   return cells_term<T, R, MODE, TZ, ES, true>(a, d, nbatch, st);
+}
+
+// Applies of a star and one diagonal of axes 0 and 1 (OpDesc::slope).
+template <typename T, int R, int SLOPE>
+cudaError_t cells_slope(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  return cells_term<T, R, MODE_APPLY, 32, (int)sizeof(T), true, SLOPE>(a, d, nbatch, st);
+}
+template <typename T>
+cudaError_t cells_diagonal(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
+  switch (d.R * d.slope) {
+    case 1: return cells_slope<T, 1, 1>(a, d, nbatch, st);
+    case 2: return cells_slope<T, 2, 1>(a, d, nbatch, st);
+    case 3: return cells_slope<T, 3, 1>(a, d, nbatch, st);
+    case -1: return cells_slope<T, 1, -1>(a, d, nbatch, st);
+    case -2: return cells_slope<T, 2, -1>(a, d, nbatch, st);
+    case -3: return cells_slope<T, 3, -1>(a, d, nbatch, st);
+  }
+  return cudaErrorInvalidValue;
 }
 
 // Tile widths: the one of the two whose tiles stage fewer cells for the grid

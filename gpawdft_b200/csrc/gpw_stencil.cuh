@@ -696,6 +696,7 @@ __global__ void __launch_bounds__(MehrCfg::NT, 2) mehrstellen_kernel(const Stenc
 struct StarCoefs {
   double cx[13], cy[13], cz[13];  // per-axis coefficients indexed offset + R (centres zero)
   double cc;                      // total centre (diagonal) coefficient
+  double cd[13];                  // the one diagonal of axes 0 and 1 (OpDesc::slope): offsets (q, slope q, 0)
 };
 
 // The same coefficients in the kernel's scalar type, rounded once on the host
@@ -705,6 +706,7 @@ template <typename S>
 struct StarCoefsT {
   S cx[13], cy[13], cz[13];
   S cc;
+  S cd[13];
 };
 template <typename S>
 inline StarCoefsT<S> star_coefs_typed(const StarCoefs& sc) {
@@ -713,6 +715,7 @@ inline StarCoefsT<S> star_coefs_typed(const StarCoefs& sc) {
     t.cx[i] = (S)sc.cx[i];
     t.cy[i] = (S)sc.cy[i];
     t.cz[i] = (S)sc.cz[i];
+    t.cd[i] = (S)sc.cd[i];
   }
   t.cc = (S)sc.cc;
   return t;

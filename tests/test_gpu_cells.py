@@ -99,3 +99,37 @@ def test_residual_and_jacobi(cuda, n, pbc, dtype, nn):
         x = ends[k].astype(float)
         oop.relax(2, x, src[k], 3, 0.7)
         assert relerr(_ends(g)[k], x) < 4 * TOL[np.dtype(dtype)]
+
+
+@pytest.mark.parametrize('nn', [1, 2, 3])
+@pytest.mark.parametrize('dtype', [np.complex128, np.complex64])
+@pytest.mark.parametrize('slope', [-1, 1])
+@pytest.mark.parametrize('n,pbc', [((20, 20, 33), (1, 1, 1)),
+                                   ((9, 9, 64), (1, 1, 0)),
+                                   ((37, 37, 12), (0, 0, 1)),
+                                   ((6, 6, 6), (1, 1, 1))])
+def test_star_and_one_diagonal(cuda, n, pbc, slope, dtype, nn):
+    """Hexagonal cells (both angles) of complex grids: the diagonal of axes 0
+    and 1 with the star, corners past one and two boundaries."""
+    import torch
+    from gpawdft_b200.fd_operators import Laplace
+    from gpawdft_b200.grid_descriptor import GridDescriptor
+    N = tuple(m if p else m + 1 for m, p in zip(n, pbc))
+    a = 0.2 * N[0]
+    cell = [(a, 0, 0), (slope * -0.5 * a, 0.75 ** 0.5 * a, 0),
+            (0, 0, 0.2 * N[2])]
+    gd, ogd = GridDescriptor(N, cell, pbc), OGD(N, cell, pbc)
+    x = rand((3,) + n, dtype, 31 * nn)
+    v = rand(n, np.float64 if dtype == np.complex128 else np.float32, 5)
+    ph = phase_cd_for_k(ogd, np.array([0.13, -0.31, 0.22]))
+    tol = TOL[np.dtype(dtype)]
+    dev, vt = torch.from_numpy(x).cuda(), torch.from_numpy(v).cuda()
+    out = torch.empty_like(dev)
+    op = Laplace(gd, -0.5, nn, dtype)
+    ref = _apply(ol.Laplace(ogd, -0.5, nn, oracle_dtype(dtype)), x, dtype, ph)
+    op.apply(dev, out, ph)
+    assert relerr(out.cpu().numpy(), ref) < tol
+    op.apply_fused(dev, out, ph, vt_g=vt, aux=dev, aux_scale=0.75)
+    assert relerr(out.cpu().numpy(), ref + x * v + 0.75 * x) < tol
+    op.apply_potential(dev, out, vt, ph)
+    assert relerr(out.cpu().numpy(), ref + x * v) < tol
