@@ -22,7 +22,7 @@ namespace gpw {
 constexpr int DIRECT_NT = 256;
 
 template <typename T, int R, int MODE>
-__global__ void __launch_bounds__(DIRECT_NT) star_direct_kernel(const StencilArgs a,
+__global__ void __launch_bounds__(DIRECT_NT, (!EltTraits<T>::cpx && R <= 3 ? 4 : 1)) star_direct_kernel(const StencilArgs a,
                                                                 const StarCoefsT<typename EltTraits<T>::S> k) {
   using S = typename EltTraits<T>::S;
   __shared__ double red[32];
