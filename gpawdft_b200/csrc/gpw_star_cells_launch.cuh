@@ -20,6 +20,13 @@ inline bool cells16_ok(const StencilArgs& a, size_t es, int nbatch) {
          (v.s0 * (int64_t)es) % 16 == 0 && (nbatch == 1 || (v.sb * (int64_t)es) % 16 == 0);
 }
 
+// Equal coefficients at +q and -q on every axis.
+inline bool star_symmetric(const StarCoefs& sc, int R) {
+  for (int q = 1; q <= R; ++q)
+    if (sc.cx[R + q] != sc.cx[R - q] || sc.cy[R + q] != sc.cy[R - q] || sc.cz[R + q] != sc.cz[R - q]) return false;
+  return true;
+}
+
 template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM, int SLOPE>
 cudaError_t cells_run(StencilArgs a, const OpDesc& d, int nbatch, cudaStream_t st) {
   using C = CellsCfg<T, R, MODE, TZ, CELLB>;

@@ -214,10 +214,7 @@ __device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigne
                : "memory");
 }
 
-// SYM: equal coefficients at +q and -q on every axis (a Laplacian): 3R + 1
-// coefficients fit in uniform registers, where 6R + 1 are loaded again on
-// every plane.
-template <typename S, int R, int MODE, int VAR, bool SYM>
+template <typename S, int R, int MODE, int VAR>
 __global__ void __launch_bounds__(TmaCfg<S, R, MODE, VAR>::NT, TmaCfg<S, R, MODE, VAR>::MINB)
     star_tma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_rho,
                     const __grid_constant__ CUtensorMap tmap_aux, const TmaArgs ta, const TmaCoefs<S> k) {
@@ -396,15 +393,15 @@ __global__ void __launch_bounds__(TmaCfg<S, R, MODE, VAR>::NT, TmaCfg<S, R, MODE
 #pragma unroll
               for (int e = 0; e < VEC; e += 2) {
                 fma_pair(k.cy[R + q], col[j + R + q].v[e], col[j + R + q].v[e + 1], p[e], p[e + 1]);
-                fma_pair(k.cy[SYM ? R + q : R - q], col[j + R - q].v[e], col[j + R - q].v[e + 1], p[e], p[e + 1]);
+                fma_pair(k.cy[R - q], col[j + R - q].v[e], col[j + R - q].v[e + 1], p[e], p[e + 1]);
                 if (q % 2 == 0) {
                   fma_pair(k.cz[R + q], nb[XL + e + q], nb[XL + e + 1 + q], pz[e], pz[e + 1]);
-                  fma_pair(k.cz[SYM ? R + q : R - q], nb[XL + e - q], nb[XL + e + 1 - q], pz[e], pz[e + 1]);
+                  fma_pair(k.cz[R - q], nb[XL + e - q], nb[XL + e + 1 - q], pz[e], pz[e + 1]);
                 } else {
 #pragma unroll
                   for (int f = e; f < e + 2; ++f) {
                     pz[f] = fma(k.cz[R + q], nb[XL + f + q], pz[f]);
-                    pz[f] = fma(k.cz[SYM ? R + q : R - q], nb[XL + f - q], pz[f]);
+                    pz[f] = fma(k.cz[R - q], nb[XL + f - q], pz[f]);
                   }
                 }
               }
@@ -431,7 +428,7 @@ __global__ void __launch_bounds__(TmaCfg<S, R, MODE, VAR>::NT, TmaCfg<S, R, MODE
                 if (m == R)
                   add_pair(p[e], p[e + 1], acc[j][pm].v[e], acc[j][pm].v[e + 1]);
                 else
-                  fma_pair(k.cx[SYM && m > R ? m : 2 * R - m], c.v[e], c.v[e + 1], acc[j][pm].v[e], acc[j][pm].v[e + 1]);
+                  fma_pair(k.cx[2 * R - m], c.v[e], c.v[e + 1], acc[j][pm].v[e], acc[j][pm].v[e + 1]);
               }
             }
           }

@@ -64,26 +64,19 @@ inline int tma_model_chunks(int n0, int64_t tiles, int R, int64_t slots) {
 
 inline int tma_max_chunks(int n0, int R) { return std::max(1, n0 / (2 * R + 2)); }
 
-// Equal coefficients at +q and -q on every axis.
-inline bool star_symmetric(const StarCoefs& sc, int R) {
-  for (int q = 1; q <= R; ++q)
-    if (sc.cx[R + q] != sc.cx[R - q] || sc.cy[R + q] != sc.cy[R - q] || sc.cz[R + q] != sc.cz[R - q]) return false;
-  return true;
-}
-
-template <typename S, int R, int MODE, int VAR, bool SYM>
+template <typename S, int R, int MODE, int VAR>
 struct TmaKernel {
   using C = TmaCfg<S, R, MODE, VAR>;
   static int slots_per_sm() {
     static int n = -1;
     static std::once_flag once;
     std::call_once(once, [] {
-      if (smem_optin_bytes(star_tma_kernel<S, R, MODE, VAR, SYM>, C::smem) != cudaSuccess) {
+      if (smem_optin_bytes(star_tma_kernel<S, R, MODE, VAR>, C::smem) != cudaSuccess) {
         n = 0;
         return;
       }
       int b = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, star_tma_kernel<S, R, MODE, VAR, SYM>, C::NT, C::smem) !=
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, star_tma_kernel<S, R, MODE, VAR>, C::NT, C::smem) !=
           cudaSuccess)
         b = 0;
       n = b;
@@ -130,7 +123,7 @@ struct TmaKernel {
       a.nblk_seg = 0;
       TmaArgs ta{a, device_status_word()};
       const TmaCoefs<S> kc = tma_coefs<S>(sc, R, a.w, a.c0, a.w2);
-      return launch_pdl(star_tma_kernel<S, R, MODE, VAR, SYM>, dim3((unsigned)nblk, 1, 1), dim3(C::NTX, C::NTY), C::smem,
+      return launch_pdl(star_tma_kernel<S, R, MODE, VAR>, dim3((unsigned)nblk, 1, 1), dim3(C::NTX, C::NTY), C::smem,
                         st, map_in, map_rho, map_aux, ta, kc);
     }
     a.split_npl = 0;
@@ -144,7 +137,7 @@ struct TmaKernel {
     a.nblk_seg = grid.x * grid.y * nc;
     TmaArgs ta{a, device_status_word()};
     const TmaCoefs<S> kc = tma_coefs<S>(sc, R, a.w, a.c0, a.w2);
-    return launch_pdl(star_tma_kernel<S, R, MODE, VAR, SYM>, grid, dim3(C::NTX, C::NTY), C::smem, st, map_in, map_rho,
+    return launch_pdl(star_tma_kernel<S, R, MODE, VAR>, grid, dim3(C::NTX, C::NTY), C::smem, st, map_in, map_rho,
                       map_aux, ta, kc);
   }
 };
@@ -153,30 +146,27 @@ template <typename S, int R, int MODE>
 cudaError_t tma_run_variant(int var, const StencilArgs& a, int nbatch, const StarCoefs& sc, int nchunk,
                             cudaStream_t st) {
   if (!tma_variant_compiled<S>(R, var)) return cudaErrorInvalidValue;
-  // other stencils than Laplacians: the default tile whatever the variant
-  if (!star_symmetric(sc, R))
-    return TmaKernel<S, R, MODE, tma_default_variant(R), false>::run(a, nbatch, sc, nchunk, st);
   if constexpr (R == 1 || R == 3) {
     switch (var) {
-      case 0: return TmaKernel<S, R, MODE, 0, true>::run(a, nbatch, sc, nchunk, st);
-      case 1: return TmaKernel<S, R, MODE, 1, true>::run(a, nbatch, sc, nchunk, st);
-      case 2: return TmaKernel<S, R, MODE, 2, true>::run(a, nbatch, sc, nchunk, st);
-      case 3: return TmaKernel<S, R, MODE, 3, true>::run(a, nbatch, sc, nchunk, st);
-      case 4: return TmaKernel<S, R, MODE, 4, true>::run(a, nbatch, sc, nchunk, st);
-      case 10: return TmaKernel<S, R, MODE, 10, true>::run(a, nbatch, sc, nchunk, st);
+      case 0: return TmaKernel<S, R, MODE, 0>::run(a, nbatch, sc, nchunk, st);
+      case 1: return TmaKernel<S, R, MODE, 1>::run(a, nbatch, sc, nchunk, st);
+      case 2: return TmaKernel<S, R, MODE, 2>::run(a, nbatch, sc, nchunk, st);
+      case 3: return TmaKernel<S, R, MODE, 3>::run(a, nbatch, sc, nchunk, st);
+      case 4: return TmaKernel<S, R, MODE, 4>::run(a, nbatch, sc, nchunk, st);
+      case 10: return TmaKernel<S, R, MODE, 10>::run(a, nbatch, sc, nchunk, st);
     }
     if constexpr (sizeof(S) == 4) {
       switch (var) {
-        case 5: return TmaKernel<S, R, MODE, 5, true>::run(a, nbatch, sc, nchunk, st);
-        case 6: return TmaKernel<S, R, MODE, 6, true>::run(a, nbatch, sc, nchunk, st);
-        case 7: return TmaKernel<S, R, MODE, 7, true>::run(a, nbatch, sc, nchunk, st);
-        case 8: return TmaKernel<S, R, MODE, 8, true>::run(a, nbatch, sc, nchunk, st);
-        case 9: return TmaKernel<S, R, MODE, 9, true>::run(a, nbatch, sc, nchunk, st);
+        case 5: return TmaKernel<S, R, MODE, 5>::run(a, nbatch, sc, nchunk, st);
+        case 6: return TmaKernel<S, R, MODE, 6>::run(a, nbatch, sc, nchunk, st);
+        case 7: return TmaKernel<S, R, MODE, 7>::run(a, nbatch, sc, nchunk, st);
+        case 8: return TmaKernel<S, R, MODE, 8>::run(a, nbatch, sc, nchunk, st);
+        case 9: return TmaKernel<S, R, MODE, 9>::run(a, nbatch, sc, nchunk, st);
       }
     }
     return cudaErrorInvalidValue;
   } else {
-    return TmaKernel<S, R, MODE, tma_default_variant(R), true>::run(a, nbatch, sc, nchunk, st);
+    return TmaKernel<S, R, MODE, tma_default_variant(R)>::run(a, nbatch, sc, nchunk, st);
   }
 }
 
