@@ -89,7 +89,7 @@ static cudaError_t run_direct(const StencilArgs& a0, const OpDesc& d, int nbatch
   const int n0 = a.vin.n[0];
   auto cost = [&](int zc) { return (col * ((n0 + zc - 1) / zc) + slots - 1) / slots * (zc + 2); };
   int best = a.zchunk;
-  for (int zc = a.zchunk + 1; zc <= std::min(n0, 4 * a.zchunk); ++zc)
+  for (int zc = a.zchunk + 1; zc <= std::min({n0, 4 * a.zchunk, a.zchunk + 32}); ++zc)
     if (cost(zc) < cost(best)) best = zc;
   a.zchunk = best;
   grid.y = (n0 + best - 1) / best;
