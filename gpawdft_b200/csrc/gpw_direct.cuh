@@ -7,8 +7,9 @@
 // march -- a chunk of planes, each a dependent load, wait and barrier -- is a
 // serial chain that takes ~10 us whatever the grid, while the grid's 1 + 6R
 // reads per point are L1 traffic a few SMs deep.  A launch here is as long as
-// one or two memory latencies.  Taken for the grids direct_ok (gpw_launch.cu)
-// names.
+// one or two memory latencies (~4 us; the V-cycles of a periodic 80^3 float64
+// solve, 28 launches each: 296 -> 146 us with this kernel and the other small-
+// grid ones).  Taken for the grids direct_ok (gpw_launch.cu) names.
 //
 // An output's in-plane terms are one chain (centre, axis 1, axis 2), as
 // c/bmgs/fd.c sums a plane; latency is hidden by the other threads.
