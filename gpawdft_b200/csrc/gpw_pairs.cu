@@ -14,7 +14,7 @@
 // rows meet in L1.
 //
 // What bounds it: the float64 rate.  48 x 48 complex128 pairs of 56^3 points
-// (3.2 GFLOP on 270 MB) take 186 us with the caller's read of the result; one
+// (3.2 GFLOP on 270 MB) take 172 us with the caller's read of the result; one
 // reduction per pair, which read every vector 48 times, took 1433 us.
 #include <algorithm>
 
