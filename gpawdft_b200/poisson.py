@@ -149,6 +149,13 @@ def inner_spectrum(operators, fine=(2, 6.0), coarsest=8):
     equal spacings (Arnoldi on the cycle: 0.79 .. 1.04 on every grid from
     32^3 to 40 x 72 x 104 points); the coarse operators' own error puts the
     smooth modes up to 1.04.
+
+    lo is at least hi / 16.  Modes below the interval are damped as well, only
+    less; but the wider the interval, the longer the longest step, and from
+    hi / lo = 25 on a cycle amplifies part of the spectrum on its way, which
+    the outer iteration takes for divergence.  At 16 no partial cycle does, nor
+    does it where the spectrum ends 6% above hi.  (A coarsest level that its
+    sweeps hardly solve, as that of 362^3, would put lo at 0 or below.)
     """
     op = operators[0]
     hi = jacobi_spectrum(op)
@@ -166,7 +173,8 @@ def inner_spectrum(operators, fine=(2, 6.0), coarsest=8):
     # 1 / T_m((top + low) / (top - low)); a single mode is solved exactly
     left = 0.0 if top - low < 1e-12 * top else \
         1.0 / np.cosh(coarsest * np.arccosh((top + low) / (top - low)))
-    return 1.0 - max(keep, left) - 0.01, 1.0 + max(left, 0.045)
+    lo, hi = 1.0 - max(keep, left) - 0.01, 1.0 + max(left, 0.045)
+    return max(lo, hi / 16), hi
 
 
 def jacobi22_schedule(L, w=2.0 / 3.0, coarsest=8):

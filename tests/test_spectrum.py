@@ -49,19 +49,41 @@ def test_star_symbol(N, pbc):
     assert abs(jacobi_spectrum(op, lowest=True) - low) < 19 * 2.0 ** -50
 
 
+def ops(N, h=(1, 1, 1), pbc=0, levels=9):
+    N = (N,) * 3 if isinstance(N, int) else N
+    gd = GridDescriptor(N, tuple(n * a for n, a in zip(N, h)), pbc)
+    out = [laplace(gd, NN3)]
+    while len(out) < levels:
+        try:
+            gd = gd.coarsen()
+        except ValueError:
+            break
+        out.append(laplace(gd, [-2.0, 1.0]))
+    return out
+
+
 def test_interval():
-    def ops(N, h=(1, 1, 1)):
-        gd = GridDescriptor((N,) * 3, tuple(N * a for a in h), 0)
-        out = [laplace(gd, NN3)]
-        while True:
-            try:
-                gd = gd.coarsen()
-            except ValueError:
-                return out
-            out.append(laplace(gd, [-2.0, 1.0]))
     lo, hi = inner_spectrum(ops(64))
     assert 0.77 < lo < 0.79 and hi == 1.045      # Arnoldi: 0.794 .. 1.042
     # unequal spacings (Arnoldi: 0.679 .. 1.056), and a 25-point coarsest level
     assert inner_spectrum(ops(32, (1, 1.15, .9)))[0] < 0.68
     lo, hi = inner_spectrum(ops(100))
     assert lo < 0.4 and hi > 1.6
+
+
+@pytest.mark.parametrize('case', [
+    dict(N=202), dict(N=354), dict(N=362), dict(N=400, levels=2),
+    dict(N=(16, 16, 1202), pbc=1)])
+def test_interval_of_hard_grids(case):
+    """Coarsest levels that their sweeps hardly solve: the engine takes the
+    interval (0 < lo < hi), and no cycle of the five step lengths amplifies a
+    mode up to 1.06 hi on its way, in the order that the engine takes them."""
+    lo, hi = inner_spectrum(ops(**case))
+    assert 0.0 < lo < hi <= 2.0
+    lam = np.linspace(0.0, 1.06 * hi, 20001)[1:]
+    p = np.ones_like(lam)
+    for j in (2, 0, 4, 1, 3):
+        node = 0.5 * (hi + lo) + 0.5 * (hi - lo) * np.cos((2 * j + 1) *
+                                                          np.pi / 10)
+        p = p * (1.0 - lam / node)
+        assert np.abs(p).max() <= 1.0
