@@ -64,12 +64,17 @@ __device__ __forceinline__ int64_t global_ns() {
 // error grew takes plain steps from there on.
 constexpr int ACCEL_M = 5;
 struct OuterAccel {
-  float* step;      // per member: the next step's length; null: plain steps
+  float* step;            // per member: the next step's length; null: plain steps
+  unsigned char* plain;   // per member: it has left the accelerated steps
   double theta, delta;
+  __device__ __forceinline__ void start(int b) const {
+    if (!step) return;
+    plain[b] = 0;
+    set(b, 0);
+  }
   // step k (from 0) of the cycle, the nodes ordered so that partial cycles
   // damp the whole interval too
   __device__ __forceinline__ void set(int b, int k) const {
-    if (!step) return;
     const int order[ACCEL_M] = {2, 0, 4, 1, 3};
     const int j = order[k % ACCEL_M];
     step[b] = (float)(1.0 / (theta + delta * cospi((2 * j + 1) / (2.0 * ACCEL_M))));
@@ -89,12 +94,13 @@ __global__ void converge_update_kernel(int nbatch, const double* __restrict__ su
   for (int b = threadIdx.x; b < nbatch; b += blockDim.x) {
     if (!active[b]) continue;
     const double e = sumsq[b] * dv;
-    // (a step of exactly 1 marks a member that has left the accelerated steps)
     if (acc.step) {
-      if (acc.step[b] != 1.f && (niter[b] == 1 || e <= err[b]))
+      if (!acc.plain[b] && (niter[b] == 1 || e <= err[b])) {
         acc.set(b, niter[b]);
-      else
+      } else {
+        acc.plain[b] = 1;
         acc.step[b] = 1.f;
+      }
     }
     err[b] = e;
     // while iterate2(step) > eps and niter < maxiter: niter += 1
@@ -124,7 +130,7 @@ __global__ void solve_setup_kernel(int nb, const double* __restrict__ h_eps, int
     eps[b] = h_eps[b];
     niter[b] = 1;
     active[b] = 1;
-    acc.set(b, 0);
+    acc.start(b);
   }
   if (threadIdx.x == 0) *maxiter_out = maxiter;
 }
@@ -195,7 +201,7 @@ struct gpw_poisson {
   bool use_rr_coarse = true;  // ... and the coarser levels' residuals
   // Chebyshev acceleration of the float32 form's outer iteration: the
   // spectrum taken for the V-cycle-preconditioned operator (hi <= lo: off),
-  // and the per-member step lengths
+  // and per member the step length and whether it takes plain steps
   double accel_lo = 0.0, accel_hi = 0.0;
   Workspace d_step;
   Workspace d_err, d_eps, d_niter, d_active, d_any, d_r64, d_gs_old, d_maxiter, d_tdone, d_t0;
@@ -802,7 +808,7 @@ static int ensure_f32(gpw_poisson* ps) {
     for (Workspace* w : {&L.phi32[0], &L.phi32[1], &L.rho32, &L.res32}) cudaMemset(w->ptr, 0, w->bytes);
   }
   if (ps->accel_hi > ps->accel_lo && fused_dc(ps) && !ps->d_step.ptr) {
-    const int rc = ps->d_step.ensure((size_t)ps->nbmax * sizeof(float));
+    const int rc = ps->d_step.ensure((size_t)ps->nbmax * (sizeof(float) + 1));
     if (rc) return rc;
     cudaMemset(ps->d_step.ptr, 0, ps->d_step.bytes);  // (finite for a tuning pass before any solve)
   }
@@ -824,6 +830,7 @@ static OuterAccel outer_accel(const gpw_poisson* ps) {
   OuterAccel a{};
   if (ps->accel_hi > ps->accel_lo && fused_dc(ps) && ps->d_step.ptr) {
     a.step = (float*)ps->d_step.ptr;
+    a.plain = (unsigned char*)(a.step + ps->nbmax);
     a.theta = 0.5 * (ps->accel_lo + ps->accel_hi);
     a.delta = 0.5 * (ps->accel_hi - ps->accel_lo);
   }
