@@ -180,6 +180,34 @@ __global__ void add_f32_kernel(int64_t n, const float* __restrict__ e, double* _
 
 using namespace gpw;
 
+// Graphs of gpw_poisson_solve_many, which hold the buffers and settings of
+// several engines: dropped when one of those is freed or (form
+// `prec_from` and up) changed.
+struct MultiKey {
+  std::vector<const void*> eng;
+  std::vector<int> nb;
+  int prec;
+  bool operator<(const MultiKey& o) const {
+    if (prec != o.prec) return prec < o.prec;
+    if (eng != o.eng) return eng < o.eng;
+    return nb < o.nb;
+  }
+};
+static std::mutex g_multi_mu;
+static std::map<MultiKey, cudaGraphExec_t> g_multi;
+static void discard_multi(const void* ps, int prec_from) {
+  std::lock_guard<std::mutex> lock(g_multi_mu);
+  for (auto it = g_multi.begin(); it != g_multi.end();) {
+    const auto& eng = it->first.eng;
+    if (it->first.prec >= prec_from && std::find(eng.begin(), eng.end(), ps) != eng.end()) {
+      cudaGraphExecDestroy(it->second);
+      it = g_multi.erase(it);
+    } else {
+      ++it;
+    }
+  }
+}
+
 struct gpw_poisson {
   std::vector<Level> lv;
   int relax_method = 2;
@@ -230,6 +258,7 @@ struct gpw_poisson {
   int64_t last_kernels = 0, last_graphs = 0;
   bool device_loop = true;  // use the device-side loop when it can be built
   ~gpw_poisson() {
+    discard_multi(this, 0);
     for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
     for (auto& kv : loops)
       if (kv.second) cudaGraphExecDestroy(kv.second);
@@ -1253,20 +1282,7 @@ extern "C" int gpw_poisson_last_latency(gpw_poisson* ps, int64_t nbatch, double*
 // Several engines (e.g. one per grid size) solved by ONE graph launch: a
 // parent graph with one device-side while loop per engine; the loops are
 // independent branches and run concurrently.  Arguments are per engine as
-// in gpw_poisson_solve.  Cached per (engines, batch sizes, form).
-struct MultiKey {
-  std::vector<const void*> eng;
-  std::vector<int> nb;
-  int prec;
-  bool operator<(const MultiKey& o) const {
-    if (prec != o.prec) return prec < o.prec;
-    if (eng != o.eng) return eng < o.eng;
-    return nb < o.nb;
-  }
-};
-static std::mutex g_multi_mu;
-static std::map<MultiKey, cudaGraphExec_t> g_multi;
-
+// in gpw_poisson_solve.  Cached per (engines, batch sizes, form) in g_multi.
 extern "C" int gpw_poisson_solve_many(int nengines, gpw_poisson* const* engines, double* const* phis,
                                       const double* const* rhos, const int64_t* nbatch,
                                       const double* const* eps, int maxiter, int precision, int* const* niters,
@@ -1342,6 +1358,7 @@ extern "C" int gpw_poisson_solve_many(int nengines, gpw_poisson* const* engines,
 // discarded.
 // Drop the captured graphs of the float32 form (its schedule or launch plan changed).
 static void discard_f32_graphs(gpw_poisson* ps) {
+  discard_multi(ps, 1);
   for (auto it = ps->graphs.begin(); it != ps->graphs.end();) {
     if (it->first.prec == 1) {
       cudaGraphExecDestroy(it->second);

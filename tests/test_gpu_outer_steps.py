@@ -98,6 +98,37 @@ def test_back_to_plain_steps(cuda):
     assert _same(phi, plain)
 
 
+def test_solve_many_takes_new_settings(cuda):
+    """Several engines in one graph: a changed interval reaches the next
+    solve, and engines made after others of the same sizes were freed have
+    graphs of their own."""
+    from gpawdft_b200 import _lib
+    from gpawdft_b200.poisson import solve_many
+    counts = []
+    for _ in range(3):
+        pairs = [_solver((N,) * 3, (.38,) * 3, 'fp32') for N in (32, 40)]
+        rhos = [_charges(gd, gd.N_c) for gd, ps in pairs]
+        eps = [1e-20 * (r ** 2).sum(axis=(1, 2, 3)) * gd.dv
+               for r, (gd, ps) in zip(rhos, pairs)]
+
+        def solve():
+            phis = [np.zeros_like(r) for r in rhos]
+            return phis, solve_many([ps for gd, ps in pairs], phis, rhos, eps)
+        fast, nfast = solve()
+        for gd, ps in pairs:
+            _lib.check(ps._lib.gpw_poisson_set_acceleration(ps._engine[0],
+                                                            0.0, 0.0))
+        plain, nplain = solve()
+        for a, b, n, m in zip(fast, plain, nfast, nplain):
+            assert (n < m).all(), (n, m)
+            assert _same(a, b)
+        counts.append(np.concatenate(nfast + nplain))
+        for gd, ps in pairs:
+            ps._free_engine()
+    assert np.array_equal(counts[0], counts[1])
+    assert np.array_equal(counts[0], counts[2])
+
+
 def test_rejects_bad_intervals(cuda):
     from gpawdft_b200 import _lib
     lib = _lib.load()
