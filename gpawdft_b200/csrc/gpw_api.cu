@@ -43,6 +43,28 @@ Workspace::~Workspace() {
   if (ptr) cudaFree(ptr);
 }
 
+int GraphScratch::get(size_t bytes) {
+  cudaError_t e = cudaMallocAsync(&ptr, bytes, st);
+  if (e == cudaSuccess) return GPW_OK;
+  ptr = nullptr;
+  return cuda_fail(e, "workspace allocation");
+}
+GraphScratch::~GraphScratch() {
+  if (ptr) cudaFreeAsync(ptr, st);
+}
+
+// What scratch a call on `st` takes: of its graph (captured), or of its device
+// and stream.
+static int scratch_place(cudaStream_t st, bool& captured, int& dev, unsigned long long& id) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(st, &cs);
+  captured = cs != cudaStreamCaptureStatusNone;
+  if (captured) return GPW_OK;  // (a capturing stream does not tell its id)
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaStreamGetId(st, &id);
+  return e == cudaSuccess ? GPW_OK : cuda_fail(e, "stream query");
+}
+
 int SumScratch::ensure(int64_t nseg, int64_t nblk_seg) {
   const bool grow_counter = (size_t)nseg * sizeof(unsigned) > counter.bytes;
   int rc = partial.ensure((size_t)(nseg * nblk_seg) * sizeof(double));
@@ -50,7 +72,9 @@ int SumScratch::ensure(int64_t nseg, int64_t nblk_seg) {
   rc = counter.ensure((size_t)nseg * sizeof(unsigned));
   if (rc) return rc;
   if (grow_counter) {
+    // (done before a stream that does not wait for the default one uses them)
     cudaError_t e = cudaMemset(counter.ptr, 0, counter.bytes);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) return cuda_fail(e, "counter init");
   }
   return result.ensure((size_t)nseg * sizeof(double));
@@ -463,21 +487,42 @@ int gpw_add_scalar(int dtype, int64_t n, double c, const void* x, void* y, gpw_s
   return e == cudaSuccess ? GPW_OK : cuda_fail(e, "add_scalar");
 }
 
+// Partials, counters (zero) and results of a segmented sum launched on
+// `graph`'s stream.
+static int sum_scratch(GraphScratch& graph, int64_t nseg, int64_t nblk_seg, GridSum& gs) {
+  bool captured;
+  int dev;
+  unsigned long long id;
+  int rc = scratch_place(graph.st, captured, dev, id);
+  if (rc) return rc;
+  if (!captured) {
+    SumScratch& scratch = stream_scratch<SumScratch>(dev, id);
+    rc = scratch.ensure(nseg, nblk_seg);
+    gs = scratch.gs();
+    return rc;
+  }
+  if ((rc = graph.get((size_t)nseg * ((nblk_seg + 1) * sizeof(double) + sizeof(unsigned))))) return rc;
+  gs.partial = (double*)graph.ptr;
+  gs.result = gs.partial + nseg * nblk_seg;
+  gs.counter = (unsigned*)(gs.result + nseg);
+  cudaError_t e = cudaMemsetAsync(gs.counter, 0, (size_t)nseg * sizeof(unsigned), graph.st);
+  return e == cudaSuccess ? GPW_OK : cuda_fail(e, "counter init");
+}
+
 static int reduce_common(int dtype, int op, int64_t nvec, int64_t n, const void* x, const void* y, double* out,
                          gpw_stream stream) {
   if (!valid_dtype(dtype) || nvec <= 0 || n <= 0 || !x || !out || nvec > 65535)
     return fail(GPW_EINVAL, "reduction: bad arguments");
-  static thread_local SumScratch scratch;
   const int nblk = reduce_blocks(n);
   const int ncomp = (op != 1 && is_complex(dtype)) ? 2 : 1;
-  int rc = scratch.ensure(nvec * ncomp, nblk);
-  if (rc) return rc;
-  GridSum gs = scratch.gs();
   cudaStream_t st = (cudaStream_t)stream;
+  GraphScratch graph(st);
+  GridSum gs;
+  int rc = sum_scratch(graph, nvec * ncomp, nblk, gs);
+  if (rc) return rc;
+  gs.result = out;
   cudaError_t e = launch_reduce(dtype, op, nvec, n, x, y, gs, nblk, st);
-  if (e != cudaSuccess) return cuda_fail(e, "reduction launch");
-  e = cudaMemcpyAsync(out, gs.result, sizeof(double) * nvec * ncomp, cudaMemcpyDeviceToDevice, st);
-  return e == cudaSuccess ? GPW_OK : cuda_fail(e, "reduction copy");
+  return e == cudaSuccess ? GPW_OK : cuda_fail(e, "reduction launch");
 }
 
 int gpw_sum(int dtype, int64_t nvec, int64_t n, const void* x, double* out_dev, gpw_stream stream) {
@@ -498,12 +543,12 @@ int gpw_poisson_charge_prepare(int64_t nb, int64_t n, const double* rho, double*
   if (rho_out == rho) return fail(GPW_EINVAL, "charge_prepare: rho_out must not alias rho");
   if ((rho_gauss == nullptr) != (phi_gauss == nullptr))
     return fail(GPW_EINVAL, "charge_prepare: give both Gaussian arrays or neither");
-  static thread_local SumScratch scratch;
   const int nblk = reduce_blocks(n);
-  int rc = scratch.ensure(nb, nblk);
-  if (rc) return rc;
-  GridSum gs = scratch.gs();
   cudaStream_t st = (cudaStream_t)stream;
+  GraphScratch graph(st);
+  GridSum gs;
+  int rc = sum_scratch(graph, nb, nblk, gs);
+  if (rc) return rc;
   cudaError_t e = launch_reduce(GPW_F64, 0, nb, n, rho, nullptr, gs, nblk, st);
   if (e != cudaSuccess) return cuda_fail(e, "charge_prepare: reduction");
   const int all_p = (pbc_mask & 7) == 7, any_p = (pbc_mask & 7) != 0;
@@ -598,10 +643,25 @@ int gpw_dotc_pairs(int dtype, int64_t nx, int64_t ny, int64_t n, const void* x, 
   // share their vectors (one launch per pair read them from L2 again)
   if (nx * ny == 1) return reduce_common(dtype, 2, 1, n, x, y, out_dev, stream);
   if (!valid_dtype(dtype) || n <= 0 || !x || !out_dev) return fail(GPW_EINVAL, "reduction: bad arguments");
-  static thread_local Workspace scratch;
-  int rc = scratch.ensure(pair_scratch_bytes(dtype, nx, ny, n));
+  cudaStream_t st = (cudaStream_t)stream;
+  GraphScratch graph(st);
+  bool captured;
+  int dev;
+  unsigned long long id;
+  int rc = scratch_place(st, captured, dev, id);
   if (rc) return rc;
-  cudaError_t e = launch_pairs(dtype, nx, ny, n, x, y, (double*)scratch.ptr, out_dev, (cudaStream_t)stream);
+  const size_t bytes = pair_scratch_bytes(dtype, nx, ny, n);
+  void* partial;
+  if (captured) {
+    rc = graph.get(bytes);
+    partial = graph.ptr;
+  } else {
+    Workspace& scratch = stream_scratch<Workspace>(dev, id);
+    rc = scratch.ensure(bytes);
+    partial = scratch.ptr;
+  }
+  if (rc) return rc;
+  cudaError_t e = launch_pairs(dtype, nx, ny, n, x, y, (double*)partial, out_dev, st);
   return e == cudaSuccess ? GPW_OK : cuda_fail(e, "reduction launch");
 }
 

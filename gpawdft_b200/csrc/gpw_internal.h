@@ -5,6 +5,8 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -217,6 +219,49 @@ struct SumScratch {
     g.result = (double*)result.ptr;
     return g;
   }
+};
+
+// Scratch of the calls that keep none in a handle (W: Workspace, SumScratch).
+// Work on one stream is ordered, so a thread keeps one W per (device, stream)
+// for the last KEEP of them and every call on another stream has another one.
+// Streams go by their id, which a later stream does not take over.  Not for
+// a capture, whose graph may run on any stream at any time: GraphScratch.
+template <typename W>
+W& stream_scratch(int dev, unsigned long long id) {
+  constexpr size_t KEEP = 8;
+  struct Entry {
+    int dev;
+    unsigned long long id;
+    std::unique_ptr<W> w;
+  };
+  static thread_local std::vector<Entry> kept;  // the last used one first
+  size_t i = 0;
+  while (i < kept.size() && (kept[i].dev != dev || kept[i].id != id)) ++i;
+  if (i == kept.size()) {
+    if (kept.size() >= KEEP) {
+      // (the calls that used it may still run)
+      cudaSetDevice(kept.back().dev);
+      cudaDeviceSynchronize();
+      cudaSetDevice(dev);
+      kept.pop_back();
+      --i;
+    }
+    kept.push_back(Entry{dev, id, std::make_unique<W>()});
+  }
+  std::rotate(kept.begin(), kept.begin() + i, kept.begin() + i + 1);
+  return *kept.front().w;
+}
+
+// Scratch of one captured call: the graph's own memory, taken by a node
+// before the call's launches and given back by one after them.
+struct GraphScratch {
+  void* ptr = nullptr;
+  cudaStream_t st;
+  explicit GraphScratch(cudaStream_t stream) : st(stream) {}
+  int get(size_t bytes);
+  GraphScratch(const GraphScratch&) = delete;
+  GraphScratch& operator=(const GraphScratch&) = delete;
+  ~GraphScratch();
 };
 
 int num_sms();
