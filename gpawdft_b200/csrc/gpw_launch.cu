@@ -251,10 +251,24 @@ static cudaError_t dispatch_mode(const StencilArgs& a, const OpDesc& d, int nbat
 
 static bool star_radius_ok(int R) { return R >= 1 && R <= 4; }
 
-static bool star_has_axis0(const OpDesc& d) {
-  for (int i = 0; i <= 2 * d.R; ++i)
-    if (d.sc.cx[i] != 0.0) return true;
-  return false;
+// The stencils that the whole-row kernel takes by rule: without terms along
+// axis 0 it stages no halo planes and keeps no sums; with terms along axis 0
+// alone it stages no halo rows or columns, but keeps 2R + 1 sums a row, which
+// pays for complex elements only.  Gradients with R = 3 of 12 to 64 grids past
+// 8 MB, us on the cell-staged kernel / this one: along axis 1 complex128 90 x
+// 82 x 65 246 / 95 and 64 x 50 x 180 122 / 90, complex64 90 x 82 x 65 269 / 145,
+// float64 95^3 83 / 71 and 93 x 70 x 45 84 / 41, float32 95^3 116 / 110 (slower
+// only float32 rows of 181 points, 117 / 123); along axis 0 complex128 246 / 97
+// and 122 / 53, complex64 268 / 147, but float64 19 x 59 x 31 18 / 20 and
+// float32 95^3 116 / 132.
+static bool rows_rule(const OpDesc& d, int dtype) {
+  if (!d.star) return false;
+  bool x = false, yz = false;
+  for (int i = 0; i <= 2 * d.R; ++i) {
+    x = x || d.sc.cx[i] != 0.0;
+    yz = yz || d.sc.cy[i] != 0.0 || d.sc.cz[i] != 0.0;
+  }
+  return !x || (!yz && is_complex(dtype));
 }
 
 // The cp.async star / general kernel for an apply (the periodic TMA row
@@ -495,10 +509,8 @@ cudaError_t launch_stencil(const OpDesc& d, int dtype, int mode, const void* in,
   }
   if (mode == MODE_APPLY && !active && bloch_path_ok(d, dtype, in, vin, out, vout, nbatch))
     return launch_bloch(d, dtype, a, nbatch, st);
-  // no axis-0 terms (a gradient): the whole-row kernel, which then stages no
-  // halo planes and keeps no sums
   if (mode == MODE_APPLY && !active && !pot && !aux && !direct_ok(a.vin, nbatch, elt_size(dtype)) &&
-      !star_has_axis0(d) && rows_ok(d, dtype, a, 4))
+      rows_rule(d, dtype) && rows_ok(d, dtype, a, 4))
     return launch_rows(d, dtype, a, nbatch, 4, st);
   OpDesc dd = d;
   if (!star_radius_ok(dd.R)) {
