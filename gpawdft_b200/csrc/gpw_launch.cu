@@ -236,9 +236,16 @@ static cudaError_t dispatch_star(const StencilArgs& a, const OpDesc& d, int nbat
   return cudaErrorInvalidValue;
 }
 
+// Planes whose bytes the cell-staged kernel's 32-bit offsets reach; larger ones
+// are served as general stencils, which keep 64-bit ones (offsets in cells,
+// widened at each copy, cost the kernel 2% at 64 x 84 x 90 x 108 complex64,
+// 423 -> 433 us).
+static bool cells_plane_ok(const GridView& v, size_t es) { return v.s0 * (int64_t)es <= UINT32_MAX; }
+
 template <typename T, int MODE>
 static cudaError_t dispatch_mode(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
   const bool use_star = (MODE == MODE_JACOBI) ? d.star_jacobi : d.star;
+  if (!cells_plane_ok(a.vin, sizeof(T))) return run_general<T, MODE>(a, d, nbatch, st);
   if (use_star) return dispatch_star<T, MODE>(a, d, nbatch, st);
   // complex bands of a hexagonal cell: the star kernel with the diagonal's
   // terms (24 x 60^2 x 84 complex128, 25 points: 118 us against 251 for the
@@ -296,16 +303,16 @@ int stencil_blocks_per_member(const OpDesc& d, int mode, const GridView& v, int 
     choose_chunks(v.n[0], (int64_t)gx * gy * nbatch, minz, zc, nc);
     return gx * gy * nc;
   };
-  int nblk;
+  int nblk = 0;
   if (use_star) {
     int zc;
     const dim3 g = direct_grid(v, nbatch, zc);
     nblk = direct_ok(v, nbatch, 4) ? (int)(g.x * g.y) : 0;
     // cell-staged tiles: at least 32 points wide and 20 rows high
     nblk = std::max(nblk, (v.n[2] + 31) / 32 * ((v.n[1] + 19) / 20) * std::max(1, v.n[0] / (2 * d.R + 2)));
-  } else {
+  }
+  if (!use_star || !cells_plane_ok(v, 16)) {
     // the tile depends on the element size: the most CTAs over the op's types
-    nblk = 0;
     for (size_t es : d.real ? std::initializer_list<size_t>{4, 8} : std::initializer_list<size_t>{8, 16}) {
       int tz, ty;
       bool blocked;

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(CellsCfg<T, R, MODE, TZ, CELLB>::NT, (R <= 3 ?
 
   // ---- this thread's cells: tid + k NT of the box.  Cells past a zero
   // boundary are never copied: they are zeroed once in every stage.
-  unsigned off[C::NLD];              // bytes from the plane's start
+  unsigned off[C::NLD];              // bytes from the plane's start (cells_plane_ok)
   unsigned valid = 0, wrapped = 0;   // bit k: inside or an image; an image along axis 1 or 2
   unsigned char side[C::NLD];        // sides + 1: bits 0-1 axis 1, bits 2-3 axis 2
 #pragma unroll

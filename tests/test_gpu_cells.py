@@ -133,3 +133,44 @@ def test_star_and_one_diagonal(cuda, n, pbc, slope, dtype, nn):
     assert relerr(out.cpu().numpy(), ref + x * v + 0.75 * x) < tol
     op.apply_potential(dev, out, vt, ph)
     assert relerr(out.cpu().numpy(), ref + x * v) < tol
+
+
+def _rows_of_five_points(op, a, n):
+    """(row, the sum of the five points in the plane) at rows of a."""
+    import torch
+    c = {tuple(o): w for o, w in zip(op.offset_pc, op.coef_p)}
+    for y in (0, 1, n // 2, n - 40, n - 1):
+        rows = torch.nn.functional.pad(a[0, max(0, y - 1):y + 2],
+                                       (1, 1, int(y == 0), int(y == n - 1)))
+        yield y, c[0, 0, 0] * rows[1, 1:-1] + \
+            c[0, 0, 1] * (rows[1, 2:] + rows[1, :-2]) + \
+            c[0, 1, 0] * (rows[0, 1:-1] + rows[2, 1:-1])
+
+
+@pytest.mark.parametrize('dtype,N', [(complex, 16500), (float, 23300)])
+def test_planes_past_32_bits(cuda, dtype, N):
+    """Planes of more than 4 GiB with rows off the 16-byte boundaries of the
+    TMA kernel: applies, and the residual with its norm."""
+    import torch
+    from gpawdft_b200.fd_operators import Laplace
+    from gpawdft_b200.grid_descriptor import GridDescriptor
+    gd = GridDescriptor((2, N, N), (0.4, 0.2 * N, 0.2 * N), 0)
+    n = N - 1
+    assert n * n * np.dtype(dtype).itemsize > 2 ** 32
+    torch.manual_seed(1)
+    a = torch.randn((1, n, n), device='cuda', dtype=torch.complex128
+                    if dtype is complex else torch.float64)
+    op = Laplace(gd, -0.5, 1, dtype)
+    out = torch.empty_like(a)
+    op.apply(a, out, None if dtype is float else np.ones((3, 2), complex))
+    for y, ref in _rows_of_five_points(op, a, n):
+        err = (out[0, y] - ref).abs().max() / ref.abs().max()
+        assert err < TOL[np.dtype(dtype)], (y, err)
+    if dtype is float:
+        norm = op.residual(a[None], a[None], out[None])
+        for y, ref in _rows_of_five_points(op, a, n):
+            ref = ref - a[0, y]
+            err = (out[0, y] - ref).abs().max() / ref.abs().max()
+            assert err < TOL[np.dtype(dtype)], (y, err)
+        want = (out * out).sum()
+        assert (norm[0] - want).abs() < 1e-12 * want
