@@ -54,13 +54,22 @@ static void choose_chunks(int n0, int64_t tiles, int minz, int& zchunk, int& nch
 static int wave_chunks(int n, int64_t tiles, int warm, int64_t slots, int maxc);
 
 // ------------------------------------------------------------------ stencils
-// Grids served by star_direct_kernel: all members together at most
-// DIRECT_BYTES of input (they stay in L2, and the marching kernels' chains of
-// planes cannot fill the chip).
+// Grids served by star_direct_kernel: all members together at most this many
+// bytes of input (they stay in L2, and the marching kernels' chains of planes
+// cannot fill the chip).  Time of the cell-staged kernel over the direct one's,
+// applies, residuals and sweeps of random grids, by millions of points: radius 1
+// 1.2 to 2.8 up to 1.2, 1.0 above; radius 2 and 3 float32 1.3 up to 0.5, 0.9
+// above 0.6, float64 1.2 at 1.0, 0.8 to 1.05 above, complex64 1.0 at 1.0,
+// complex128 1.15 at 0.5, 0.9 above; radius 4 float32 0.9 above 0.6, float64
+// 1.25 at 0.7, 0.93 at 1.0, complex64 1.2 at 0.5, 0.6 above, complex128 1.2 at
+// 0.3, 0.86 at 0.5.
 constexpr int64_t DIRECT_BYTES = 8 << 20;
-static bool direct_ok(const GridView& v, int64_t nbatch, size_t es) {
-  return (int64_t)v.n[0] * v.n[1] * v.n[2] * nbatch * (int64_t)es <= DIRECT_BYTES && nbatch <= 65535 &&
-         v.s0 <= INT32_MAX;
+static int64_t direct_bytes(size_t es, int R) {
+  if (R == 1) return DIRECT_BYTES;
+  return es == 4 ? 5 << 19 : (R >= 4 ? 5 << 20 : DIRECT_BYTES);
+}
+static bool direct_ok(const GridView& v, int64_t nbatch, size_t es, int64_t most = DIRECT_BYTES) {
+  return (int64_t)v.n[0] * v.n[1] * v.n[2] * nbatch * (int64_t)es <= most && nbatch <= 65535 && v.s0 <= INT32_MAX;
 }
 // its grid: 256 points of a plane and a run of planes per CTA, about 8 CTAs
 // per SM
@@ -100,7 +109,7 @@ static cudaError_t run_direct(const StencilArgs& a0, const OpDesc& d, int nbatch
 
 template <typename T, int R, int MODE>
 static cudaError_t run_star(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
-  if (direct_ok(a.vin, nbatch, sizeof(T))) return run_direct<T, R, MODE>(a, d, nbatch, st);
+  if (direct_ok(a.vin, nbatch, sizeof(T), direct_bytes(sizeof(T), R))) return run_direct<T, R, MODE>(a, d, nbatch, st);
   if constexpr (EltTraits<T>::cpx) {
     static_assert(MODE == MODE_APPLY, "complex grids: applies only");
     return sizeof(T) == 16 ? launch_cells_c128(a, d, nbatch, st) : launch_cells_c64(a, d, nbatch, st);
@@ -308,8 +317,8 @@ int stencil_blocks_per_member(const OpDesc& d, int mode, const GridView& v, int 
     int zc;
     const dim3 g = direct_grid(v, nbatch, zc);
     nblk = direct_ok(v, nbatch, 4) ? (int)(g.x * g.y) : 0;
-    // cell-staged tiles: at least 32 points wide and 20 rows high
-    nblk = std::max(nblk, (v.n[2] + 31) / 32 * ((v.n[1] + 19) / 20) * std::max(1, v.n[0] / (2 * d.R + 2)));
+    // cell-staged tiles: at least 32 points wide and 16 rows high
+    nblk = std::max(nblk, (v.n[2] + 31) / 32 * ((v.n[1] + 15) / 16) * std::max(1, v.n[0] / (2 * d.R + 2)));
   }
   if (!use_star || !cells_plane_ok(v, 16)) {
     // the tile depends on the element size: the most CTAs over the op's types

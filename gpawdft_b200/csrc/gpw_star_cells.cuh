@@ -9,7 +9,7 @@
 //    a zero boundary are zeroed once, periodic ones have wrapped sources, and
 //    Bloch phases are a fix-up of the thread's own wrapped cells.
 //  * A thread owns 16 bytes of adjacent axis-2 scalars (1 complex128, 2
-//    complex64 or float64, 4 float32 elements) x PY rows and reads shared
+//    complex64 or float64, 4 float32 elements) x PY (1 or 2) rows and reads shared
 //    memory in 16-byte vectors at compile-time offsets.  Complex data is the
 //    scalar stencil with axis-2 offsets doubled.
 //  * One CTA barrier per plane: the load that refills a stage is issued after
@@ -35,14 +35,14 @@
 
 namespace gpw {
 
-// TZ: tile width in elements; CELLB: bytes per staged cell.
-template <typename T, int R, int MODE, int TZ_, int CELLB>
+// TZ: tile width in elements; CELLB: bytes per staged cell; PY: rows a thread.
+template <typename T, int R, int MODE, int TZ_, int CELLB, int PY_ = 2>
 struct CellsCfg {
   using S = typename EltTraits<T>::S;
   static constexpr int ES = (int)sizeof(T), CS = EltTraits<T>::cpx ? 2 : 1;
   static constexpr int VEC = 16 / (int)sizeof(S);         // scalars per thread
   static constexpr int EPT = VEC / CS;                    // elements per thread
-  static constexpr int TZ = TZ_, NTX = TZ / EPT, PY = 2;
+  static constexpr int TZ = TZ_, NTX = TZ / EPT, PY = PY_;
   static constexpr int NTY = 256 / NTX, NT = NTX * NTY, TY = NTY * PY;
   static constexpr int AL = 16 / ES;                      // elements per 16 bytes
   static constexpr int XL = (R + AL - 1) / AL * AL;       // halo columns, whole vectors
@@ -53,6 +53,8 @@ struct CellsCfg {
   static constexpr int D = 3, NS = D + 1 + JR;            // planes in flight, stages
   static constexpr int STAGE = (H * W * ES + 127) / 128 * 128;
   static constexpr size_t smem = (size_t)NS * STAGE;
+  // CTAs per SM the registers must allow
+  static constexpr int MINB = R == 1 && PY == 1 ? (sizeof(S) == 4 ? 3 : 4) : 2;
 };
 
 // EPI: an apply with a potential (1: a.pot) or an aux term (2: a.aux, and
@@ -66,12 +68,12 @@ struct CellsCfg {
 // ones, so that fewer partial sums of its size are rounded (60^2 x 84 normal
 // values, R = 3: error against extended precision 1.3e-16; 1.8e-16 with the
 // centre first, 2.3e-16 for the general kernel's order).
-template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM, int SLOPE>
-__global__ void __launch_bounds__(CellsCfg<T, R, MODE, TZ, CELLB>::NT, (R <= 3 ? 2 : 1))
+template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM, int SLOPE, int PY = 2>
+__global__ void __launch_bounds__(CellsCfg<T, R, MODE, TZ, CELLB, PY>::NT, (CellsCfg<T, R, MODE, TZ, CELLB, PY>::MINB))
     star_cells_kernel(const StencilArgs a, const StarCoefsT<typename EltTraits<T>::S> k) {
-  using C = CellsCfg<T, R, MODE, TZ, CELLB>;
+  using C = CellsCfg<T, R, MODE, TZ, CELLB, PY>;
   using S = typename EltTraits<T>::S;
-  constexpr int VEC = C::VEC, CS = C::CS, EPT = C::EPT, PY = C::PY, NR = 2 * R + 1, NS = C::NS, NT = C::NT;
+  constexpr int VEC = C::VEC, CS = C::CS, EPT = C::EPT, NR = 2 * R + 1, NS = C::NS, NT = C::NT;
   constexpr int WS = C::W * CS, XS = C::XL * CS;  // row pitch and halo in scalars
   using P = Pack<S, VEC>;
   extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -27,10 +27,10 @@ inline bool star_symmetric(const StarCoefs& sc, int R) {
   return true;
 }
 
-template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM, int SLOPE>
+template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, bool SYM, int SLOPE, int PY>
 cudaError_t cells_run(StencilArgs a, const OpDesc& d, int nbatch, cudaStream_t st) {
-  using C = CellsCfg<T, R, MODE, TZ, CELLB>;
-  auto kern = star_cells_kernel<T, R, MODE, TZ, CELLB, EPI, SYM, SLOPE>;
+  using C = CellsCfg<T, R, MODE, TZ, CELLB, PY>;
+  auto kern = star_cells_kernel<T, R, MODE, TZ, CELLB, EPI, SYM, SLOPE, PY>;
   static std::once_flag once;
   static cudaError_t oe = cudaSuccess;
   static int per_sm = 1;
@@ -49,20 +49,20 @@ cudaError_t cells_run(StencilArgs a, const OpDesc& d, int nbatch, cudaStream_t s
   return launch_pdl(kern, grid, dim3(C::NT), C::smem, st, a, star_coefs_typed<typename EltTraits<T>::S>(d.sc));
 }
 
-template <typename T, int R, int MODE, int TZ, int CELLB, bool SYM, int SLOPE = 0>
+template <typename T, int R, int MODE, int TZ, int CELLB, bool SYM, int SLOPE = 0, int PY = 2>
 cudaError_t cells_term(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
   if constexpr (MODE == MODE_APPLY) {
-    if (a.aux) return cells_run<T, R, MODE, TZ, CELLB, 2, SYM, SLOPE>(a, d, nbatch, st);
-    if (a.pot) return cells_run<T, R, MODE, TZ, CELLB, 1, SYM, SLOPE>(a, d, nbatch, st);
+    if (a.aux) return cells_run<T, R, MODE, TZ, CELLB, 2, SYM, SLOPE, PY>(a, d, nbatch, st);
+    if (a.pot) return cells_run<T, R, MODE, TZ, CELLB, 1, SYM, SLOPE, PY>(a, d, nbatch, st);
   }
-  return cells_run<T, R, MODE, TZ, CELLB, 0, SYM, SLOPE>(a, d, nbatch, st);
+  return cells_run<T, R, MODE, TZ, CELLB, 0, SYM, SLOPE, PY>(a, d, nbatch, st);
 }
 
-template <typename T, int R, int MODE, int TZ>
+template <typename T, int R, int MODE, int TZ, int PY>
 cudaError_t cells_form(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
   constexpr int ES = (int)sizeof(T);
-  if (ES < 16 && cells16_ok(a, ES, nbatch)) return cells_term<T, R, MODE, TZ, 16, true>(a, d, nbatch, st);
-  return cells_term<T, R, MODE, TZ, ES, true>(a, d, nbatch, st);
+  if (ES < 16 && cells16_ok(a, ES, nbatch)) return cells_term<T, R, MODE, TZ, 16, true, 0, PY>(a, d, nbatch, st);
+  return cells_term<T, R, MODE, TZ, ES, true, 0, PY>(a, d, nbatch, st);
 }
 
 // Applies of a star and one diagonal of axes 0 and 1 (OpDesc::slope).
@@ -83,23 +83,38 @@ cudaError_t cells_diagonal(const StencilArgs& a, const OpDesc& d, int nbatch, cu
   return cudaErrorInvalidValue;
 }
 
-// Tile widths: the one of the two whose tiles stage fewer cells for the grid
-// (radius 1 and 3, the stencils of GPAW's levels; one width for the others).
+// Tiles: 64 x 32 points for float32, 32 x 16 for complex128, else 32 x 32, with
+// two rows a thread; for radius 1 and 3 (the stencils of GPAW's levels) also 48
+// (complex128 24) points wide; and 32 wide with one row a thread for float32
+// (32 x 32: narrow grids leave fewer lanes of it empty) and, of the 8-byte
+// types, for radius 1 (more CTAs per SM) and 4 (two, where two rows a thread
+// allow one).  Of these the one with the least work: staged cells, and twice
+// its points (one row a thread: 1.6 times).  us with the two-row tiles alone /
+// with this choice: a residual of 796 x 61 x 32 x 19 float32, radius 3, 441 /
+// 205, of 329 x 14 x 48 x 73 float64, radius 1, 134 / 109, a Laplacian of 70 x
+// 24 x 72 x 37 complex64, radius 4, 174 / 125.
 template <typename T, int R, int MODE>
 cudaError_t cells_width(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
-  constexpr int TA = sizeof(T) == 4 ? 64 : 32, TB = sizeof(T) == 16 ? 24 : 48;
-  // other stencils than Laplacians: one width and cell size
-  if (!star_symmetric(d.sc, R)) return cells_term<T, R, MODE, TA, (int)sizeof(T), false>(a, d, nbatch, st);
-  if constexpr (R == 1 || R == 3) {
-    using CA = CellsCfg<T, R, MODE, TA, (int)sizeof(T)>;
-    using CB = CellsCfg<T, R, MODE, TB, (int)sizeof(T)>;
-    auto cells = [&](int tz, int ty, int box) {
-      return (int64_t)((a.vout.n[2] + tz - 1) / tz) * ((a.vout.n[1] + ty - 1) / ty) * box;
-    };
-    if (cells(TB, CB::TY, CB::H * CB::W) < cells(TA, CA::TY, CA::H * CA::W))
-      return cells_form<T, R, MODE, TB>(a, d, nbatch, st);
+  constexpr int ES = (int)sizeof(T), TA = ES == 4 ? 64 : 32, TB = ES == 16 ? 24 : 48;
+  constexpr bool ONE = ES == 4 || (ES == 8 && (R == 1 || R == 4)), WIDE = R == 1 || R == 3;
+  // other stencils than Laplacians: one tile and cell size
+  if (!star_symmetric(d.sc, R)) return cells_term<T, R, MODE, 32, ES, false, 0, ES == 4 ? 1 : 2>(a, d, nbatch, st);
+  auto work = [&](auto cfg) {
+    using C = decltype(cfg);
+    const int64_t tiles = (int64_t)((a.vout.n[2] + C::TZ - 1) / C::TZ) * ((a.vout.n[1] + C::TY - 1) / C::TY);
+    return (double)tiles * (C::H * C::W + (C::PY == 1 ? 1.6 : 2.0) * C::TZ * C::TY);
+  };
+  const double wa = work(CellsCfg<T, R, MODE, TA, ES, 2>());
+  double wb = 1e300, wc = 1e300;
+  if constexpr (WIDE) wb = work(CellsCfg<T, R, MODE, TB, ES, 2>());
+  if constexpr (ONE) wc = work(CellsCfg<T, R, MODE, 32, ES, 1>());
+  if constexpr (ONE) {
+    if (wc < wa && wc < wb) return cells_form<T, R, MODE, 32, 1>(a, d, nbatch, st);
   }
-  return cells_form<T, R, MODE, TA>(a, d, nbatch, st);
+  if constexpr (WIDE) {
+    if (wb < wa) return cells_form<T, R, MODE, TB, 2>(a, d, nbatch, st);
+  }
+  return cells_form<T, R, MODE, TA, 2>(a, d, nbatch, st);
 }
 
 template <typename T, int MODE>

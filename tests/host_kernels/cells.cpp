@@ -29,9 +29,9 @@ struct Guarded {
   void* at(bool high) const { return map + G + (high ? len - bytes : 0); }
 };
 
-template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, int SLOPE>
+template <typename T, int R, int MODE, int TZ, int CELLB, int EPI, int SLOPE, int PY = 2>
 static void walk(int n0, int n1, int n2, int nb, int nchunk, bool pot, bool aux, bool periodic) {
-  using C = CellsCfg<T, R, MODE, TZ, CELLB>;
+  using C = CellsCfg<T, R, MODE, TZ, CELLB, PY>;
   using S = typename EltTraits<T>::S;
   const size_t pts = (size_t)n0 * n1 * n2;
   Guarded in(pts * nb * sizeof(T)), out(pts * nb * sizeof(T)), other(pts * nb * sizeof(T)), v(pts * sizeof(S));
@@ -54,16 +54,16 @@ static void walk(int n0, int n1, int n2, int nb, int nchunk, bool pot, bool aux,
       for (blockIdx.y = 0; blockIdx.y < gridDim.y; ++blockIdx.y)
         for (blockIdx.x = 0; blockIdx.x < gridDim.x; ++blockIdx.x)
           for (threadIdx.x = 0; threadIdx.x < blockDim.x; ++threadIdx.x)
-            star_cells_kernel<T, R, MODE, TZ, CELLB, EPI, true, SLOPE>(a, StarCoefsT<S>{});
+            star_cells_kernel<T, R, MODE, TZ, CELLB, EPI, true, SLOPE, PY>(a, StarCoefsT<S>{});
   }
 }
 
-template <typename T, int R, int TZ, int CELLB, int SLOPE>
+template <typename T, int R, int TZ, int CELLB, int SLOPE, int PY = 2>
 static void applies(int n0, int n1, int n2, int nb, int nchunk, bool periodic) {
-  walk<T, R, MODE_APPLY, TZ, CELLB, 0, SLOPE>(n0, n1, n2, nb, nchunk, false, false, periodic);
-  walk<T, R, MODE_APPLY, TZ, CELLB, 1, SLOPE>(n0, n1, n2, nb, nchunk, true, false, periodic);
-  walk<T, R, MODE_APPLY, TZ, CELLB, 2, SLOPE>(n0, n1, n2, nb, nchunk, false, true, periodic);
-  walk<T, R, MODE_APPLY, TZ, CELLB, 2, SLOPE>(n0, n1, n2, nb, nchunk, true, true, periodic);
+  walk<T, R, MODE_APPLY, TZ, CELLB, 0, SLOPE, PY>(n0, n1, n2, nb, nchunk, false, false, periodic);
+  walk<T, R, MODE_APPLY, TZ, CELLB, 1, SLOPE, PY>(n0, n1, n2, nb, nchunk, true, false, periodic);
+  walk<T, R, MODE_APPLY, TZ, CELLB, 2, SLOPE, PY>(n0, n1, n2, nb, nchunk, false, true, periodic);
+  walk<T, R, MODE_APPLY, TZ, CELLB, 2, SLOPE, PY>(n0, n1, n2, nb, nchunk, true, true, periodic);
 }
 
 int main() {
@@ -74,6 +74,9 @@ int main() {
     applies<double, 3, 32, 8, 0>(17, 33, 31, 2, 2, periodic);
     applies<double, 2, 48, 16, 0>(12, 21, 50, 1, 2, periodic);
     applies<double, 4, 32, 8, 0>(3, 3, 3, 1, 1, periodic);
+    applies<double, 4, 32, 16, 0, 1>(11, 17, 34, 1, 1, periodic);
+    applies<float, 2, 32, 4, 0, 1>(13, 33, 37, 2, 2, periodic);
+    applies<float2, 1, 32, 8, 0, 1>(9, 17, 31, 2, 2, periodic);
     walk<double, 3, MODE_RESIDUAL, 32, 8, 0, 0>(17, 33, 31, 2, 2, false, false, periodic);
     walk<double, 1, MODE_JACOBI, 48, 16, 0, 0>(9, 21, 50, 2, 2, false, false, periodic);
   }

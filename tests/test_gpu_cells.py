@@ -2,7 +2,7 @@
 (c/operators.c apply, c/bmgs/relax.c, c/bmgs/fd.c restated): batches just past
 the size up to which the small-grid kernel serves (8 MB of input), with rows
 of odd length (one element a cell) and of whole 16-byte units, partial tiles
-in both axes and both tile widths, every radius, every mix of periodic and
+in both axes and every tile, every radius, every mix of periodic and
 zero axes, Bloch phases, and the potential, aux, residual and Jacobi
 epilogues.  The first and last members are compared; tolerances as for the
 other stencils (float32 sums of squares: 1e-6)."""
@@ -18,7 +18,8 @@ pytestmark = pytest.mark.gpu
 DTYPES = [np.complex128, np.complex64, np.float64, np.float32]
 CASES = [((23, 49, 51), (0, 0, 0)), ((23, 49, 51), (1, 1, 1)),
          ((9, 45, 64), (1, 1, 1)), ((21, 35, 96), (0, 1, 1)),
-         ((12, 130, 33), (1, 0, 1))]
+         ((12, 130, 33), (1, 0, 1)), ((11, 19, 22), (1, 1, 0)),
+         ((9, 47, 67), (0, 1, 1))]
 
 
 def _setup(n, pbc, dtype, seed):
