@@ -128,18 +128,32 @@ static void general_tile(int mp, size_t es, int& tz, int& ty, bool& blocked) {
   ty = blocked ? bty : GEN_TY;
 }
 
-// Opt kernel `kern` in to `smem` bytes of dynamic shared memory (the
-// largest so far; the static part counts against the same per-CTA limit).
-template <typename K>
-static cudaError_t general_optin(K kern, size_t smem, std::mutex& mu, size_t& opted) {
-  std::lock_guard<std::mutex> lock(mu);
-  if (smem > opted) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    opted = smem;
+// A general kernel's shared-memory opt-in (to the largest size so far; the
+// static part counts against the same per-CTA limit) and its CTAs per SM by
+// size.
+struct GeneralKernel {
+  std::mutex mu;
+  size_t opted = 48 * 1024;
+  std::map<size_t, int> per_sm;
+  template <typename K>
+  cudaError_t prepare(K kern, int threads, size_t smem, int& ctas) {
+    std::lock_guard<std::mutex> lock(mu);
+    if (smem > opted) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      opted = smem;
+    }
+    auto it = per_sm.find(smem);
+    if (it == per_sm.end()) {
+      int n = 0;
+      cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem);
+      if (e != cudaSuccess) return e;
+      it = per_sm.emplace(smem, std::max(1, n)).first;
+    }
+    ctas = it->second;
+    return cudaSuccess;
   }
-  return cudaSuccess;
-}
+};
 
 // The operator is the Mehrstellen Laplacian A: 19 coefficients at exactly
 // the offsets of MEHR_OFF, in that order.
@@ -193,14 +207,7 @@ static cudaError_t run_general(const StencilArgs& a0, const OpDesc& d, int nbatc
   general_tile(mp, sizeof(T), tz, ty, blocked);
   if (blocked && (tz != GenBlk<T, 1>::TZ || ty != GenBlk<T, 1>::TY)) return cudaErrorInvalidConfiguration;
   dim3 grid((v.n[2] + tz - 1) / tz, (v.n[1] + ty - 1) / ty, 1);
-  // (chunks for whole waves of two CTAs per SM, each chunk paying 2mp planes
-  // again; the norm's partial slots count the chunks choose_chunks gives)
   choose_chunks(v.n[0], (int64_t)grid.x * grid.y * nbatch, 2 * mp + 2, a.zchunk, a.nchunk);
-  const int nc = wave_chunks(v.n[0], (int64_t)grid.x * grid.y * nbatch, 2 * mp, 2LL * num_sms(), a.nchunk);
-  a.zchunk = (v.n[0] + nc - 1) / nc;
-  a.nchunk = (v.n[0] + a.zchunk - 1) / a.zchunk;
-  grid.z = a.nchunk * nbatch;
-  a.nblk_seg = grid.x * grid.y * a.nchunk;
   // planes loaded ahead: as many (up to 4) as keep two CTAs per SM
   int depth = 1;
   while (blocked && depth < 4 && general_block_smem(mp, sizeof(T), tz, ty, d.gc.ncoef, depth + 1) <= 110 * 1024)
@@ -209,29 +216,37 @@ static cudaError_t run_general(const StencilArgs& a0, const OpDesc& d, int nbatc
   const size_t smem = blocked ? general_block_smem(mp, sizeof(T), tz, ty, d.gc.ncoef, depth)
                               : (size_t)(2 * mp + 2) * (ty + 2 * mp) * (tz + 2 * mp) * sizeof(T);
   if (smem > 227 * 1024) return cudaErrorInvalidValue;
+  // fewer chunks where they fill the waves of `kern`'s resident CTAs better,
+  // each chunk paying 2mp planes again (the norm's partial slots count the
+  // chunks choose_chunks gives).  Laplacians of fcc cells, us with choose_chunks'
+  // chunks / waves of two CTAs per SM / of the resident ones: 37 x 56^3 float32,
+  // radius 2, 69 / 94 / 68, 20 x 104^3 float64, radius 1, 234 / 307 / 234, 22 x 53^3
+  // complex64, radius 3, 248 / 167 / 167.
+  auto go = [&](auto kern, dim3 block, GeneralKernel& k) -> cudaError_t {
+    int per_sm = 1;
+    cudaError_t e = k.prepare(kern, block.x * block.y, smem, per_sm);
+    if (e != cudaSuccess) return e;
+    const int nc = wave_chunks(v.n[0], (int64_t)grid.x * grid.y * nbatch, 2 * mp, (int64_t)per_sm * num_sms(),
+                               a.nchunk);
+    a.zchunk = (v.n[0] + nc - 1) / nc;
+    a.nchunk = (v.n[0] + a.zchunk - 1) / a.zchunk;
+    grid.z = a.nchunk * nbatch;
+    a.nblk_seg = grid.x * grid.y * a.nchunk;
+    kern<<<grid, block, smem, st>>>(a, d.gc);
+    return cudaGetLastError();
+  };
   if (blocked) {
-    auto go = [&](auto kern, std::mutex& mu, size_t& opted) -> cudaError_t {
-      cudaError_t e = general_optin(kern, smem, mu, opted);
-      if (e != cudaSuccess) return e;
-      kern<<<grid, dim3(32, GenBlk<T, 1>::NTY), smem, st>>>(a, d.gc);
-      return cudaGetLastError();
-    };
-    static std::mutex mu[GEN_BLK_MAXMP];
-    static size_t opted[GEN_BLK_MAXMP] = {48 * 1024, 48 * 1024, 48 * 1024};
+    static GeneralKernel k[GEN_BLK_MAXMP];
+    const dim3 block(32, GenBlk<T, 1>::NTY);
     switch (mp) {
-      case 1: return go(general_block_kernel<T, MODE, 1>, mu[0], opted[0]);
-      case 2: return go(general_block_kernel<T, MODE, 2>, mu[1], opted[1]);
-      case 3: return go(general_block_kernel<T, MODE, 3>, mu[2], opted[2]);
+      case 1: return go(general_block_kernel<T, MODE, 1>, block, k[0]);
+      case 2: return go(general_block_kernel<T, MODE, 2>, block, k[1]);
+      case 3: return go(general_block_kernel<T, MODE, 3>, block, k[2]);
     }
     return cudaErrorInvalidValue;
   }
-  auto kern = general_stencil_kernel<T, MODE>;
-  static std::mutex mu;
-  static size_t opted = 48 * 1024;
-  cudaError_t e = general_optin(kern, smem, mu, opted);
-  if (e != cudaSuccess) return e;
-  kern<<<grid, dim3(GEN_TZ, GEN_TY), smem, st>>>(a, d.gc);
-  return cudaGetLastError();
+  static GeneralKernel k;
+  return go(general_stencil_kernel<T, MODE>, dim3(GEN_TZ, GEN_TY), k);
 }
 
 template <typename T, int MODE>

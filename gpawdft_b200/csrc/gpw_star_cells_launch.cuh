@@ -91,7 +91,7 @@ cudaError_t cells_diagonal(const StencilArgs& a, const OpDesc& d, int nbatch, cu
 // allow one).  Of these the one with the least work: staged cells, and twice
 // its points (one row a thread: 1.6 times).  us with the two-row tiles alone /
 // with this choice: a residual of 796 x 61 x 32 x 19 float32, radius 3, 441 /
-// 205, of 329 x 14 x 48 x 73 float64, radius 1, 134 / 109, a Laplacian of 70 x
+// 189, of 329 x 14 x 48 x 73 float64, radius 1, 134 / 110, a Laplacian of 70 x
 // 24 x 72 x 37 complex64, radius 4, 174 / 125.
 template <typename T, int R, int MODE>
 cudaError_t cells_width(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
