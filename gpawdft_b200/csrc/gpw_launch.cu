@@ -764,15 +764,49 @@ static cudaError_t run_restrict(const TransferArgs& a, int nbatch, cudaStream_t 
                             nbatch, st);
 }
 
-template <typename T, int K>
-static cudaError_t run_interp(const TransferArgs& a, int nbatch, cudaStream_t st) {
-  using C = InterpCfg<T, K>;
+template <typename T, int K, int PY>
+static cudaError_t run_interp_rows(const TransferArgs& a, int nbatch, cudaStream_t st) {
+  using C = InterpCfg<T, K, PY>;
   static std::once_flag once;
   static cudaError_t oe = cudaSuccess;
   static int per_sm = 1;
   const dim3 grid((a.vout.n[2] + C::OZ - 1) / C::OZ, (a.vout.n[1] + C::OY - 1) / C::OY, 1);
-  return run_transfer_tiles(interpolate_kernel<T, K>, once, oe, per_sm, dim3(C::OZ, C::NTY), C::smem, grid,
+  return run_transfer_tiles(interpolate_kernel<T, K, PY>, once, oe, per_sm, dim3(C::OZ, C::NTY), C::smem, grid,
                             2 * (K - 1), 4, a, nbatch, st);
+}
+// Two rows a thread (tiles of 32 x 16 points); 8-byte elements with K = 6 four,
+// of grids that make 1500 such tiles of four planes and more: time of two rows
+// over four, 300 random grids, float32 0.78 - 0.96, 8-byte elements K = 2 and 4
+// 0.8, K = 6 0.85 below 900 tiles, 0.98 below 1500, 1.07 below 3000, 1.0 above (2 x
+// 191^3 float64 points 52.3 / 51.2 us); not of grids of which the wider tiles
+// cover more rows (19 x 149 x 33 x 149 float64 points 74.7 / 97.7).  Four rows of
+// K = 8, or of complex128, leave no two CTAs per SM.
+template <typename T, int K>
+static cudaError_t run_interp(const TransferArgs& a, int nbatch, cudaStream_t st) {
+  if constexpr (sizeof(T) == 8 && K == 6) {
+    const int high = (a.vout.n[1] + 31) / 32, low = (a.vout.n[1] + 15) / 16;  // tiles along axis 1
+    const int64_t tiles = (int64_t)((a.vout.n[2] + 31) / 32) * high * nbatch;
+    if (tiles * (a.vout.n[0] / 4) >= 1500 && 20 * high <= 11 * low) return run_interp_rows<T, K, 4>(a, nbatch, st);
+  }
+  return run_interp_rows<T, K, 2>(a, nbatch, st);
+}
+
+// Output planes per CTA of a K = 2 kernel that evaluates its points directly:
+// per_sm CTAs per SM, of at least `longest` planes; where those are fewer than
+// three per SM, shorter ones down to `shortest` until they are three (a small
+// grid's march is a chain of dependent loads; more chunks than that only read
+// and restrict their first planes again).  500 random grids: with chunks down
+// to the shortest at once, one real transfer in five was up to 29% slower than
+// with the long ones alone; with two, three, four CTAs per SM 13, 7, 14 of 300.
+static void k2_chunks(int n0, int64_t tiles, int per_sm, int longest, int shortest, int& zchunk, int& nchunk) {
+  auto chunks = [&](int ctas, int planes) {
+    const int64_t want = ((int64_t)ctas * num_sms() + tiles - 1) / tiles;
+    return std::max<int64_t>(1, std::min<int64_t>(want, (n0 + planes - 1) / planes));
+  };
+  int64_t nc = chunks(per_sm, longest);
+  if (tiles * nc < 3LL * num_sms()) nc = chunks(3, shortest);
+  zchunk = (int)((n0 + nc - 1) / nc);
+  nchunk = (n0 + zchunk - 1) / zchunk;
 }
 
 // Restriction layout: 0 = the launcher's choice, 1 = the tile kernel
@@ -1190,13 +1224,7 @@ cudaError_t launch_transfer(const TrDesc& d, int dtype, const void* in, const Gr
     return dtype == GPW_F64 ? run_restrict_tma<double>(a, nbatch, st) : run_restrict_tma<float>(a, nbatch, st);
   if (d.k == 2 && (dtype == GPW_F64 || dtype == GPW_F32) && !interp && k2r_vec_ok(a)) {
     dim3 grid((vout.n[2] + 2 * K2V_TX - 1) / (2 * K2V_TX), (vout.n[1] + K2V_TY - 1) / K2V_TY, 1);
-    // ~8 CTAs of 256 threads per SM; chunks of at least 2 output planes
-    const int64_t tiles = (int64_t)grid.x * grid.y * nbatch;
-    const int64_t want = 8LL * num_sms();
-    int64_t nc = std::max<int64_t>(1, (want + tiles - 1) / tiles);
-    nc = std::min<int64_t>(nc, std::max(1, vout.n[0] / 2));
-    a.zchunk = (int)((vout.n[0] + nc - 1) / nc);
-    a.nchunk = (vout.n[0] + a.zchunk - 1) / a.zchunk;
+    k2_chunks(vout.n[0], (int64_t)grid.x * grid.y * nbatch, 8, interp ? 8 : 4, 2, a.zchunk, a.nchunk);
     grid.z = a.nchunk * nbatch;
     const dim3 blk(K2V_TX, K2V_TY);
     if (dtype == GPW_F64) return launch_pdl(restrict_k2_vec_kernel<double>, grid, blk, 0, st, a);
@@ -1206,29 +1234,24 @@ cudaError_t launch_transfer(const TrDesc& d, int dtype, const void* in, const Gr
     return dtype == GPW_F64 ? run_interp_tma<double>(a, nbatch, st) : run_interp_tma<float>(a, nbatch, st);
   if (d.k == 2 && (dtype == GPW_F64 || dtype == GPW_F32) && interp && k2_vec_ok(a)) {
     dim3 grid((vout.n[2] + 4 * K2V_TX - 1) / (4 * K2V_TX), (vout.n[1] + K2V_TY - 1) / K2V_TY, 1);
-    // ~8 CTAs of 256 threads per SM; chunks of at least 2 output planes
-    const int64_t tiles = (int64_t)grid.x * grid.y * nbatch;
-    const int64_t want = 8LL * num_sms();
-    int64_t nc = std::max<int64_t>(1, (want + tiles - 1) / tiles);
-    nc = std::min<int64_t>(nc, std::max(1, vout.n[0] / 2));
-    a.zchunk = (int)((vout.n[0] + nc - 1) / nc);
-    a.nchunk = (vout.n[0] + a.zchunk - 1) / a.zchunk;
+    k2_chunks(vout.n[0], (int64_t)grid.x * grid.y * nbatch, 8, interp ? 8 : 4, 2, a.zchunk, a.nchunk);
     grid.z = a.nchunk * nbatch;
     const dim3 blk(K2V_TX, K2V_TY);
     if (dtype == GPW_F64) return launch_pdl(interpolate_k2_vec_kernel<double>, grid, blk, 0, st, a);
     return launch_pdl(interpolate_k2_vec_kernel<float>, grid, blk, 0, st, a);
   }
-  // every other K = 2 transfer of real data, and complex ones that stay in L2
-  // (18^3 x 16 complex128: 6 us instead of the tile kernels' 16 - 30; at
-  // 72^3 x 16 these take 93 and 45 us against 70 and 36) unless a test pins
-  // their restriction kernel
-  const bool small = direct_ok(interp ? vout : vin, nbatch, elt_size(dtype));
+  // every other K = 2 transfer of real data, and complex ones of little data
+  // (input of a restriction, output of an interpolation) unless a test pins
+  // their restriction kernel.  Time of the tile or row kernels over these, 400
+  // random grids: interpolations 1.07 up to 2 MB, 0.88 to 4, 0.6 - 0.8 above;
+  // restrictions of complex64 1.1 up to 8 MB, 0.98 to 16, 0.8 above, of
+  // complex128 1.4 up to 8, 1.16 to 16, 0.85 above.
+  const int64_t most = interp ? 2 << 20 : (dtype == GPW_C128 ? 16 << 20 : 8 << 20);
+  const bool small = direct_ok(interp ? vout : vin, nbatch, elt_size(dtype), most);
   if (d.k == 2 &&
       (dtype == GPW_F64 || dtype == GPW_F32 || (small && (interp || g_restrict_force.load() == 0)))) {
     dim3 grid((vout.n[2] + K2_TX - 1) / K2_TX, (vout.n[1] + K2_TY - 1) / K2_TY, 1);
-    // single planes where even those leave SMs idle: a small grid's march is
-    // a chain of dependent loads
-    choose_chunks(vout.n[0], (int64_t)grid.x * grid.y * nbatch, interp ? 2 : 1, a.zchunk, a.nchunk);
+    k2_chunks(vout.n[0], (int64_t)grid.x * grid.y * nbatch, 4, 4, interp ? 2 : 1, a.zchunk, a.nchunk);
     grid.z = a.nchunk * nbatch;
     const dim3 blk(K2_TX, K2_TY);
     switch (dtype) {

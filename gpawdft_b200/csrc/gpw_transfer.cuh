@@ -327,14 +327,10 @@ __global__ void __launch_bounds__(RestrictCfg<T, K>::NT, 2) restrict_kernel(cons
 // between the same two barriers.  A thread owns PY adjacent fine rows of one
 // column, whose axis-1 pass reads K - 1 + PY / 2 values once, and keeps K
 // axis-0 values of each.
-template <typename T, int K>
+template <typename T, int K, int PY_>
 struct InterpCfg {
   static constexpr int OZ = 32, NTY = 8, NT = OZ * NTY;
-  // rows per thread, and CTAs per SM the registers must allow (4 rows of K
-  // axis-0 values do not fit two CTAs per SM for complex128 from K = 4 on
-  // and for 8-byte elements at K = 8)
-  static constexpr int PY = (sizeof(T) * K >= 64) ? 2 : 4;
-  static constexpr int MINB = (sizeof(T) * K >= 128) ? 1 : 2;
+  static constexpr int PY = PY_;  // rows per thread
   static constexpr int OY = NTY * PY, NM = PY / 2;
   static constexpr int H = OY / 2 + K - 1;     // coarse rows per plane tile
   static constexpr int W = OZ / 2 + K;         // coarse cols
@@ -342,11 +338,12 @@ struct InterpCfg {
   static constexpr size_t smem = (size_t)(NS * H * W + 2 * H * OZ) * sizeof(T);
 };
 
-template <typename T, int K>
-__global__ void __launch_bounds__(InterpCfg<T, K>::NT, (InterpCfg<T, K>::MINB)) interpolate_kernel(const TransferArgs a) {
-  using C = InterpCfg<T, K>;
+template <typename T, int K, int PY>
+__global__ void __launch_bounds__(InterpCfg<T, K, PY>::NT, (sizeof(T) * K >= 128 ? 1 : 2))
+    interpolate_kernel(const TransferArgs a) {
+  using C = InterpCfg<T, K, PY>;
   using S = typename EltTraits<T>::S;
-  constexpr int H = C::H, W = C::W, NS = C::NS, PY = C::PY, NM = C::NM, OZ = C::OZ, NT = C::NT;
+  constexpr int H = C::H, W = C::W, NS = C::NS, NM = C::NM, OZ = C::OZ, NT = C::NT;
   constexpr int base = K / 2 - 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* ring = reinterpret_cast<T*>(smem_raw);
