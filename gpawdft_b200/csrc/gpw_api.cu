@@ -510,7 +510,7 @@ static int sum_scratch(GraphScratch& graph, int64_t nseg, int64_t nblk_seg, Grid
 }
 
 static int reduce_common(int dtype, int op, int64_t nvec, int64_t n, const void* x, const void* y, double* out,
-                         gpw_stream stream) {
+                         gpw_stream stream, int ny = 1) {
   if (!valid_dtype(dtype) || nvec <= 0 || n <= 0 || !x || !out || nvec > 65535)
     return fail(GPW_EINVAL, "reduction: bad arguments");
   const int nblk = reduce_blocks(n);
@@ -521,7 +521,7 @@ static int reduce_common(int dtype, int op, int64_t nvec, int64_t n, const void*
   int rc = sum_scratch(graph, nvec * ncomp, nblk, gs);
   if (rc) return rc;
   gs.result = out;
-  cudaError_t e = launch_reduce(dtype, op, nvec, n, x, y, gs, nblk, st);
+  cudaError_t e = launch_reduce(dtype, op, nvec, n, x, y, gs, nblk, st, ny);
   return e == cudaSuccess ? GPW_OK : cuda_fail(e, "reduction launch");
 }
 
@@ -639,9 +639,14 @@ int gpw_dotc_pairs(int dtype, int64_t nx, int64_t ny, int64_t n, const void* x, 
                    gpw_stream stream) {
   if (!y) return fail(GPW_EINVAL, "null argument");
   if (nx <= 0 || ny <= 0 || nx * ny > 65535) return fail(GPW_EINVAL, "dotc_pairs: 1 <= nx * ny <= 65535");
-  // a single pair reads each vector once: the plain reduction; several pairs
-  // share their vectors (one launch per pair read them from L2 again)
-  if (nx * ny == 1) return reduce_common(dtype, 2, 1, n, x, y, out_dev, stream);
+  // few pairs of long vectors: one reduction a pair (a single one reads each
+  // vector once; several find them in L2).  Time of the tensor-core kernel,
+  // whose 8 x 8 blocks they leave mostly empty, over it, replayed from a graph
+  // (which adds ~2 us to the reductions, for their zeroed counters): above 60000
+  // points up to 16 pairs 1.25 - 1.6, to 32 1.1 - 1.5, to 64 0.9 (float64) -
+  // 1.2; at 20000 to 60000 0.8 - 1.3, to 64 0.9; below 20000 0.5 - 0.85.
+  if (nx * ny == 1 || (nx * ny <= 32 && n >= 32768))
+    return reduce_common(dtype, 2, nx * ny, n, x, y, out_dev, stream, (int)ny);
   if (!valid_dtype(dtype) || n <= 0 || !x || !out_dev) return fail(GPW_EINVAL, "reduction: bad arguments");
   cudaStream_t st = (cudaStream_t)stream;
   GraphScratch graph(st);

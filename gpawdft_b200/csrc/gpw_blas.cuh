@@ -59,15 +59,16 @@ __global__ void add_scalar_kernel(int64_t n, double c, const S* __restrict__ x, 
 // Segmented sum / dot: segment m = blockIdx.y, CTAs of one segment = gridDim.x.
 // OP 0: sum(x[m]) (real; complex -> real and imaginary in two segments),
 // OP 1: real part of sum(conj(x[m]) y[m]),
-// OP 2: sum(conj(x[m]) y[m]); complex results take two segments (real,
-//       imaginary).  Matrices over several vectors: gpw_pairs.cu.
+// OP 2: sum(conj(x[m / ny]) y[m % ny]) over every (x, y) vector pair; complex
+//       results take two segments (real, imaginary).  Larger matrices:
+//       gpw_pairs.cu.
 template <typename T, int OP>
 __global__ void __launch_bounds__(256) reduce_kernel(int64_t n, const T* __restrict__ x,
-                                                     const T* __restrict__ y, GridSum gs, int ncomp) {
+                                                     const T* __restrict__ y, GridSum gs, int ncomp, int ny) {
   __shared__ double red[32];
   const int m = blockIdx.y;
-  const T* xv = x + (int64_t)m * n;
-  const T* yv = y ? y + (int64_t)m * n : nullptr;
+  const T* xv = x + (int64_t)(OP == 2 ? m / ny : m) * n;
+  const T* yv = y ? y + (int64_t)(OP == 2 ? m % ny : m) * n : nullptr;
   double s0 = 0.0, s1 = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     if constexpr (OP == 0) {

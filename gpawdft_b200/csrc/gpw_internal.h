@@ -172,7 +172,7 @@ cudaError_t launch_cluster_vcycle(const ClusterArgs& a, size_t smem, int nbatch,
 cudaError_t launch_axpy(int dtype, int64_t n, double ar, double ai, const void* x, void* y, cudaStream_t st);
 cudaError_t launch_scal(int dtype, int64_t n, double ar, double ai, void* x, cudaStream_t st);
 cudaError_t launch_reduce(int dtype, int op, int64_t nvec, int64_t n, const void* x, const void* y,
-                          const GridSum& gs, int nblk, cudaStream_t st);
+                          const GridSum& gs, int nblk, cudaStream_t st, int ny = 1);
 // the matrix of nx * ny dot products (gpw_pairs.cu): scratch bytes, and the
 // launch (out: nx * ny values, two doubles each for complex types)
 size_t pair_scratch_bytes(int dtype, int64_t nx, int64_t ny, int64_t n);

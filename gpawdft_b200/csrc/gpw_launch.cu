@@ -1325,13 +1325,13 @@ int reduce_blocks(int64_t n) {
 }
 
 cudaError_t launch_reduce(int dtype, int op, int64_t nvec, int64_t n, const void* x, const void* y,
-                          const GridSum& gs, int nblk, cudaStream_t st) {
+                          const GridSum& gs, int nblk, cudaStream_t st, int ny) {
   dim3 grid(nblk, (unsigned)nvec);
   const int ncomp = (op != 1 && is_complex(dtype)) ? 2 : 1;
 #define GPW_REDUCE_CASE(T)                                                                              \
-  if (op == 0) reduce_kernel<T, 0><<<grid, 256, 0, st>>>(n, (const T*)x, nullptr, gs, ncomp);       \
-  else if (op == 1) reduce_kernel<T, 1><<<grid, 256, 0, st>>>(n, (const T*)x, (const T*)y, gs, ncomp); \
-  else reduce_kernel<T, 2><<<grid, 256, 0, st>>>(n, (const T*)x, (const T*)y, gs, ncomp);
+  if (op == 0) reduce_kernel<T, 0><<<grid, 256, 0, st>>>(n, (const T*)x, nullptr, gs, ncomp, 1);       \
+  else if (op == 1) reduce_kernel<T, 1><<<grid, 256, 0, st>>>(n, (const T*)x, (const T*)y, gs, ncomp, 1); \
+  else reduce_kernel<T, 2><<<grid, 256, 0, st>>>(n, (const T*)x, (const T*)y, gs, ncomp, ny);
   switch (dtype) {
     case GPW_F64: GPW_REDUCE_CASE(double) break;
     case GPW_F32: GPW_REDUCE_CASE(float) break;

@@ -1,6 +1,7 @@
 """The matrix of pair integrals on the tensor-core kernel (gpw_pairs.cu)
 against NumPy in 64 bits, at the edges of its 8 x 8 blocks, warp tiles and
-point ranges, for every element type.
+point ranges, for every element type; and few pairs of long vectors, which
+take a reduction each.
 
 Bound: a sum of n products in float64, in any order, is off by at most
 n 2^-53 sum |a| |b| (complex: four real products per term)."""
@@ -17,7 +18,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize('nx,ny,N', [(1, 2, (1, 1, 1)), (2, 1, (3, 1, 1)),
                                      (7, 9, (4, 4, 4)), (8, 8, (5, 7, 9)),
                                      (24, 25, (8, 8, 1)), (17, 33, (9, 7, 31)),
-                                     (49, 3, (16, 16, 17))])
+                                     (49, 3, (16, 16, 17)), (3, 5, (40, 41, 43)),
+                                     (33, 1, (40, 41, 43))])
 def test_pair_matrix(cuda, dtype, nx, ny, N):
     from gpawdft_b200 import blas
     import torch
