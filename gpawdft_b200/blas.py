@@ -45,7 +45,7 @@ def vector_sums(x, nvec):
                            arrays.ptr(out), arrays.stream()))
     out = out.cpu().numpy()
     if ncomp == 2:
-        return out[0::2] + 1j * out[1::2]
+        return out.view(complex)
     return out
 
 
@@ -77,7 +77,7 @@ def pair_dots(x, nx, y, ny):
                                   arrays.stream()))
     out = out.cpu().numpy()
     if cplx:
-        out = out[0::2] + 1j * out[1::2]
+        out = out.view(complex)
     return out.reshape(nx, ny)
 
 

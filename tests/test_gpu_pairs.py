@@ -37,3 +37,30 @@ def test_pair_matrix(cuda, dtype, nx, ny, N):
     again = blas.pair_dots(torch.from_numpy(a).cuda(), nx,
                            torch.from_numpy(b).cuda(), ny)
     assert np.array_equal(got, again)
+
+
+@pytest.mark.parametrize('dtype', [np.float64, np.complex128, np.float32,
+                                   np.complex64])
+@pytest.mark.parametrize('value', [np.inf, -np.inf, np.nan])
+def test_not_finite(cuda, dtype, value):
+    """An infinity or NaN in one vector reaches the pairs of that vector, with
+    the sign it has there, and no other pair of its block."""
+    from gpawdft_b200 import blas
+    import torch
+    a = rand((9, 6, 7, 8), dtype, 1)
+    b = rand((11, 6, 7, 8), dtype, 2)
+    a[4, 2, 3, 1] = value
+    b[7, 5, 6, 7] = value
+    got = blas.pair_dots(torch.from_numpy(a).cuda(), 9,
+                         torch.from_numpy(b).cuda(), 11)
+    cplx = np.dtype(dtype).kind == 'c'
+    a, b = a.reshape(9, -1), b.reshape(11, -1)
+    with np.errstate(invalid='ignore'):
+        parts = [((a.real, b.real), (a.imag, b.imag)),
+                 ((a.real, b.imag), (-a.imag, b.real))][:1 + cplx]
+        ref = [sum(x.astype(float) @ y.astype(float).T
+                   for x, y in (p if cplx else p[:1])) for p in parts]
+    for g, r in zip((got.real, got.imag), ref):
+        assert np.array_equal(np.isnan(g), np.isnan(r))
+        assert np.array_equal(g[np.isinf(r)], r[np.isinf(r)])
+        assert np.isfinite(g[np.isfinite(r)]).all()
