@@ -23,8 +23,9 @@ namespace {
 
 // A tile layout: VEC points per lane, WPR warps spanning a row, NW warps
 // per CTA (TY = NW / WPR * PY rows), and the axis-0 chunking; vec == 0
-// stands for the kernel of gpw_stencil.cuh / gpw_direct.cuh, vec == -py for
-// the whole-row kernel (gpw_rows.cuh) with py rows a thread.
+// stands for the cell-staged or direct kernel (gpw_star_cells.cuh,
+// gpw_direct.cuh), vec == -py for the whole-row kernel (gpw_rows.cuh) with py
+// rows a thread.
 struct BlochChoice {
   int vec, wpr, nw;
   int nchunk;  // 0: wave model, < 0: model x -nchunk
@@ -244,8 +245,8 @@ void tune_export_bloch(std::string& out) {
 }
 
 // One "bloch ..." record back into the tuner; a layout that is not among
-// the shape's candidates (nor the cp.async kernel, vec 0, nor the whole-row
-// kernel, vec < 0) is refused.
+// the shape's candidates (nor the cell-staged or direct kernel, vec 0, nor
+// the whole-row kernel, vec < 0) is refused.
 bool tune_import_bloch(const int* f) {
   const int dtype = f[0], R = f[1];
   if (!valid_dtype(dtype) || R < 1 || R > 3 || f[3] <= 0 || f[4] <= 0 || f[5] <= 0 || f[6] <= 0) return false;
@@ -300,7 +301,7 @@ cudaError_t launch_bloch(const OpDesc& d, int dtype, const StencilArgs& sa, int 
   if (cands.empty()) return cudaErrorInvalidValue;
   auto run = [&](const BlochChoice& c) {
     if (c.vec < 0 && rows_ok(d, dtype, sa, -c.vec)) return launch_rows(d, dtype, sa, nbatch, -c.vec, st);
-    return c.vec <= 0 ? launch_apply_cpasync(d, dtype, sa, nbatch, st)
+    return c.vec <= 0 ? launch_apply_untuned(d, dtype, sa, nbatch, st)
                       : bloch_launch(dtype, d.R, c, in, vin, out, vout, nbatch, bc, d.sc, sa.pot, sa.aux,
                                      sa.aux_scale, st);
   };
@@ -332,7 +333,7 @@ cudaError_t launch_bloch(const OpDesc& d, int dtype, const StencilArgs& sa, int 
           c.nchunk = nc;
           trial.push_back(c);
         }
-      trial.push_back(BlochChoice{0, 0, 0, 0});  // the cp.async or direct kernel
+      trial.push_back(BlochChoice{0, 0, 0, 0});  // the cell-staged or direct kernel
       for (int py : {2, 4})
         if (rows_ok(d, dtype, sa, py)) trial.push_back(BlochChoice{-py, 0, 0, 0});
       for (const BlochChoice& c : trial) {

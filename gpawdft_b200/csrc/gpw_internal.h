@@ -319,8 +319,8 @@ cudaError_t launch_cells_f32(int mode, const StencilArgs& a, const OpDesc& d, in
 cudaError_t launch_cells_c128(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st);
 cudaError_t launch_cells_c64(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st);
 cudaError_t launch_rows_f32(const OpDesc& d, int dtype, const StencilArgs& sa, int nbatch, cudaStream_t st);
-// The cp.async star / general kernel for an apply.
-cudaError_t launch_apply_cpasync(const OpDesc& d, int dtype, const StencilArgs& a, int nbatch, cudaStream_t st);
+// The star or general kernel that an apply takes outside the tuned paths.
+cudaError_t launch_apply_untuned(const OpDesc& d, int dtype, const StencilArgs& a, int nbatch, cudaStream_t st);
 
 // Device status word written by kernels whose bounded waits expire
 // (GPW_ETIMEDOUT); allocated on first use, which must not happen inside a

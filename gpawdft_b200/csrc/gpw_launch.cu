@@ -273,7 +273,9 @@ static cudaError_t dispatch_mode(const StencilArgs& a, const OpDesc& d, int nbat
   if (use_star) return dispatch_star<T, MODE>(a, d, nbatch, st);
   // complex bands of a hexagonal cell: the star kernel with the diagonal's
   // terms (24 x 60^2 x 84 complex128, 25 points: 118 us against 251 for the
-  // general kernel, which reads shared memory once per output and coefficient)
+  // general kernel, which reads shared memory once per output and coefficient).
+  // Real grids stay on the general kernel, whose results equal the reference's C
+  // bit for bit; the star form of their operators is not measured.
   if constexpr (EltTraits<T>::cpx && MODE == MODE_APPLY) {
     if (d.slope) return sizeof(T) == 16 ? launch_cells_c128(a, d, nbatch, st) : launch_cells_c64(a, d, nbatch, st);
   }
@@ -283,7 +285,8 @@ static cudaError_t dispatch_mode(const StencilArgs& a, const OpDesc& d, int nbat
 static bool star_radius_ok(int R) { return R >= 1 && R <= 4; }
 
 // The stencils that the whole-row kernel takes by rule: without terms along
-// axis 0 it stages no halo planes and keeps no sums; with terms along axis 0
+// axis 0 it stages no halo planes and keeps no sums (float32 of radius 1 is
+// faster on the cell-staged one, up to 1.6 times); with terms along axis 0
 // alone it stages no halo rows or columns, but keeps 2R + 1 sums a row, which
 // pays for complex elements only.  Gradients with R = 3 of 12 to 64 grids past
 // 8 MB, us on the cell-staged kernel / this one: along axis 1 complex128 90 x
@@ -291,20 +294,26 @@ static bool star_radius_ok(int R) { return R >= 1 && R <= 4; }
 // float64 95^3 83 / 71 and 93 x 70 x 45 84 / 41, float32 95^3 116 / 110 (slower
 // only float32 rows of 181 points, 117 / 123); along axis 0 complex128 246 / 97
 // and 122 / 53, complex64 268 / 147, but float64 19 x 59 x 31 18 / 20 and
-// float32 95^3 116 / 132.
-static bool rows_rule(const OpDesc& d, int dtype) {
-  if (!d.star) return false;
+// float32 95^3 116 / 132.  Smaller inputs take the direct kernel: its time over
+// this one's, without axis-0 terms and radius 2 to 4, 0.5 - 0.9 below 2 MB, 1.08
+// (float32) and 0.8 - 1.0 at 2 to 4, 1.1 - 1.35 at 4 to 8; radius 1 0.4 - 0.9 up to
+// 6 MB and 1.0 above, axis 0 0.3 - 0.9 and 1.0.  Returns the bytes of input past
+// which the kernel is taken.
+static int64_t rows_past(const OpDesc& d, int dtype) {
+  if (!d.star) return INT64_MAX;
   bool x = false, yz = false;
   for (int i = 0; i <= 2 * d.R; ++i) {
     x = x || d.sc.cx[i] != 0.0;
     yz = yz || d.sc.cy[i] != 0.0 || d.sc.cz[i] != 0.0;
   }
-  return !x || (!yz && is_complex(dtype));
+  if (x) return !yz && is_complex(dtype) ? DIRECT_BYTES : INT64_MAX;
+  if (d.R == 1) return dtype == GPW_F32 ? INT64_MAX : DIRECT_BYTES;
+  return dtype == GPW_F32 ? 2 << 20 : 4 << 20;
 }
 
-// The cp.async star / general kernel for an apply (the periodic TMA row
-// kernel's tuner times it beside its own layouts).
-cudaError_t launch_apply_cpasync(const OpDesc& d, int dtype, const StencilArgs& a, int nbatch, cudaStream_t st) {
+// The star or general kernel that an apply takes outside the tuned paths (the
+// periodic TMA row kernel's tuner times it beside its own layouts).
+cudaError_t launch_apply_untuned(const OpDesc& d, int dtype, const StencilArgs& a, int nbatch, cudaStream_t st) {
   OpDesc dd = d;
   if (!star_radius_ok(dd.R)) {
     dd.star = false;
@@ -540,8 +549,8 @@ cudaError_t launch_stencil(const OpDesc& d, int dtype, int mode, const void* in,
   }
   if (mode == MODE_APPLY && !active && bloch_path_ok(d, dtype, in, vin, out, vout, nbatch))
     return launch_bloch(d, dtype, a, nbatch, st);
-  if (mode == MODE_APPLY && !active && !pot && !aux && !direct_ok(a.vin, nbatch, elt_size(dtype)) &&
-      rows_rule(d, dtype) && rows_ok(d, dtype, a, 4))
+  if (mode == MODE_APPLY && !active && !pot && !aux &&
+      !direct_ok(a.vin, nbatch, elt_size(dtype), rows_past(d, dtype)) && rows_ok(d, dtype, a, 4))
     return launch_rows(d, dtype, a, nbatch, 4, st);
   OpDesc dd = d;
   if (!star_radius_ok(dd.R)) {

@@ -87,11 +87,12 @@ cudaError_t cells_diagonal(const StencilArgs& a, const OpDesc& d, int nbatch, cu
 // two rows a thread; for radius 1 and 3 (the stencils of GPAW's levels) also 48
 // (complex128 24) points wide; and 32 wide with one row a thread for float32
 // (32 x 32: narrow grids leave fewer lanes of it empty) and, of the 8-byte
-// types, for radius 1 (more CTAs per SM) and 4 (two, where two rows a thread
-// allow one).  Of these the one with the least work: staged cells, and twice
-// its points (one row a thread: 1.6 times).  us with the two-row tiles alone /
-// with this choice: a residual of 796 x 61 x 32 x 19 float32, radius 3, 441 /
-// 189, of 329 x 14 x 48 x 73 float64, radius 1, 134 / 110, a Laplacian of 70 x
+// types, for radius 1 (more CTAs per SM) and 4 (no spills).  Of these the one
+// with the least work -- staged cells, and twice its points (one row a thread:
+// 1.6 times) -- of all its CTAs or, where they leave resident slots empty, of as
+// many as there are slots.  us with the two-row tiles alone / with this choice:
+// residuals of 796 x 61 x 32 x 19 float32, radius 3, 441 / 189, of 7 x 21 x 70 x 70
+// 33 / 17, of 329 x 14 x 48 x 73 float64, radius 1, 134 / 110, a Laplacian of 70 x
 // 24 x 72 x 37 complex64, radius 4, 174 / 125.
 template <typename T, int R, int MODE>
 cudaError_t cells_width(const StencilArgs& a, const OpDesc& d, int nbatch, cudaStream_t st) {
@@ -102,7 +103,9 @@ cudaError_t cells_width(const StencilArgs& a, const OpDesc& d, int nbatch, cudaS
   auto work = [&](auto cfg) {
     using C = decltype(cfg);
     const int64_t tiles = (int64_t)((a.vout.n[2] + C::TZ - 1) / C::TZ) * ((a.vout.n[1] + C::TY - 1) / C::TY);
-    return (double)tiles * (C::H * C::W + (C::PY == 1 ? 1.6 : 2.0) * C::TZ * C::TY);
+    const int64_t ctas = tiles * nbatch * std::max(1, a.vout.n[0] / (2 * R + 2));
+    return (double)std::max<int64_t>(ctas, 2LL * num_sms()) *
+           (C::H * C::W + (C::PY == 1 ? 1.6 : 2.0) * C::TZ * C::TY);
   };
   const double wa = work(CellsCfg<T, R, MODE, TA, ES, 2>());
   double wb = 1e300, wc = 1e300;

@@ -111,29 +111,33 @@ def test_many_bands_past_l2(cuda, pin, pbc, dtype):
         assert torch.equal(out[b], one)
 
 
-@pytest.mark.parametrize('dtype', [np.complex128, np.complex64])
+@pytest.mark.parametrize('dtype', DTYPES)
 @pytest.mark.parametrize('n,pbc', [((9, 10, 31), (1, 1, 1)),
                                    ((18, 33, 65), (1, 1, 1)),
                                    ((9, 50, 180), (0, 1, 1)),
                                    ((21, 6, 32), (1, 0, 0)),
                                    ((5, 7, 250), (1, 1, 1))])
-@pytest.mark.parametrize('skew', [0, 1])
-def test_gradients_by_rule(cuda, n, pbc, dtype, skew):
-    """Complex gradients past 8 MB of grids without a tuned layout: the rule
-    that sends terms along one axis to the whole-row kernel, with rows too
-    long for it and (complex64) grids that start off a 16-byte boundary."""
+@pytest.mark.parametrize('skew,mb', [(0, 9), (1, 9), (0, 4.5), (0, 2.5)])
+@pytest.mark.parametrize('nn', [1, 3])
+def test_gradients_by_rule(cuda, n, pbc, dtype, skew, mb, nn):
+    """Gradients of grids without a tuned layout to both sides of the sizes at
+    which the rule sends them to the whole-row kernel, with rows too long for
+    it and (but complex128) grids that start off a 16-byte boundary."""
     import torch
     from gpawdft_b200.fd_operators import Gradient
     gd, ogd = _setup(n, pbc)
-    nin = 9 * 2 ** 20 // (int(np.prod(n)) * np.dtype(dtype).itemsize) + 1
+    if np.dtype(dtype) == np.dtype(complex):
+        skew = 0
+    nin = int(mb * 2 ** 20 / (int(np.prod(n)) * np.dtype(dtype).itemsize)) + 1
     size = nin * int(np.prod(n))
     flat = torch.from_numpy(rand((size + skew,), dtype, 8)).cuda()
     a = flat[skew:].view((nin,) + tuple(gd.n_c))
-    ends = a[[0, -1]].cpu().numpy().astype(complex)
+    ends = a[[0, -1]].cpu().numpy().astype(oracle_dtype(dtype))
     ph = _phases(ogd, dtype, 9)
     for axis in range(3):
         out = torch.empty_like(a)
-        Gradient(gd, axis, 1.0, 3, dtype).apply(a, out, ph)
+        Gradient(gd, axis, 1.0, nn, dtype).apply(a, out, ph)
         ref = np.zeros_like(ends)
-        ol.Gradient(ogd, axis, 1.0, 3, complex).apply(ends, ref, ph)
+        ol.Gradient(ogd, axis, 1.0, nn, oracle_dtype(dtype)).apply(ends, ref,
+                                                                   ph)
         assert relerr(out[[0, -1]].cpu().numpy(), ref) < TOL[np.dtype(dtype)]
