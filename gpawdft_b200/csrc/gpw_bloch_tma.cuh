@@ -3,8 +3,8 @@
 //
 // The band stencils of the eigensolver (Laplace / kinetic nn=3 and the
 // gradients on periodic cells, c/operators.c:316-405 with the Bloch halo of
-// c/bc.c:138-250) run here.  Compared with the cp.async kernel of
-// gpw_stencil.cuh:
+// c/bc.c:138-250) run here.  Compared with the cell-staged kernel
+// (gpw_star_cells.cuh):
 //  * a CTA owns whole rows (axis 2) of TY axis-1 rows and marches along
 //    axis 0; per plane one thread issues three 4D TMA box loads into a ring
 //    stage -- the R halo rows above, the TY rows, the R halo rows below --

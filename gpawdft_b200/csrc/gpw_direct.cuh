@@ -2,14 +2,14 @@
 // short run of axis-0 planes, every neighbour read straight from global
 // memory (L1 / L2 hits), no staging.
 //
-// The marching kernels (gpw_stencil.cuh, gpw_star_tma.cuh) read each value
+// The marching kernels (gpw_star_cells.cuh, gpw_star_tma.cuh) read each value
 // from memory once, which is what bounds large grids; on a small grid their
 // march -- a chunk of planes, each a dependent load, wait and barrier -- is a
 // serial chain that takes ~10 us whatever the grid, while the grid's 1 + 6R
 // reads per point are L1 traffic a few SMs deep.  A launch here is as long as
 // one or two memory latencies (~4 us; the V-cycles of a periodic 80^3 float64
 // solve, 28 launches each: 296 -> 146 us with this kernel and the other small-
-// grid ones).  Taken for the grids direct_ok (gpw_launch.cu) names.
+// grid ones).  Taken for the grids direct_bytes (gpw_launch.cu) names.
 //
 // An output's in-plane terms are one chain (centre, axis 1, axis 2), as
 // c/bmgs/fd.c sums a plane; latency is hidden by the other threads.

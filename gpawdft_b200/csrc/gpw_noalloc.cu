@@ -75,7 +75,7 @@ void noalloc_chunks(int n0, int64_t tiles, int minz, int& zchunk, int& nchunk) {
   nchunk = (n0 + zchunk - 1) / zchunk;
 }
 
-// Launch geometry + launch of the residual kernel on a star (cp.async) or
+// Launch geometry + launch of the residual kernel on a star (cell-staged) or
 // general-offset stencil; returns the CTAs per grid through `nblk`.
 template <typename T, int R>
 cudaError_t star_residual(StencilArgs a, const OpDesc& d, int nbatch, bool launch, int64_t& nblk,

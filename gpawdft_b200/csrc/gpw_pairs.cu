@@ -13,9 +13,12 @@
 // The warps of a CTA take adjacent tiles of the same points, so their common
 // rows meet in L1.
 //
-// What bounds it: the float64 rate.  48 x 48 complex128 pairs of 56^3 points
-// (3.2 GFLOP on 270 MB) take 172 us with the caller's read of the result; one
-// reduction per pair, which read every vector 48 times, took 1433 us.
+// What bounds it: 48 x 48 complex128 pairs of 56^3 points (3.2 GFLOP on 270 MB)
+// take 115 us, 28 TFLOP/s or about three quarters of the nominal float64 tensor
+// rate, its eight warps per SM waiting for that pipe and, less, for operands
+// (4.8 and 3.1 stall cycles an instruction in dependent and full pipes, 2.8 in
+// loads); with the sum over parts and the caller's read of the result 164 - 177
+// us.  One reduction per pair, which read every vector 48 times, took 1433 us.
 #include <algorithm>
 
 #include "gpw_internal.h"

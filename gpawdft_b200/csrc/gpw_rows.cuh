@@ -22,10 +22,10 @@
 //  * The grid is one CTA per resident slot; each takes an equal share of the
 //    (tile, plane) units, so no last wave is partly empty.
 // Measured: a gradient along axis 1 of 32 x 80 x 72 x 88 complex128, R = 3,
-// 217 us on the fastest of the other kernels, 104 us here (5.0 TB/s, 75% of the
+// 217 us on the fastest of the other kernels, 104 us here (5.0 TB/s, 77% of the
 // copy rate).  With axis-0 terms its sums per row cost more than the cell-
 // staged kernel's halo (kinetic + potential, 48 x 95^3 float64: 375 against
-// 238 us).
+// 217 us).
 // Terms are summed in the order of gpw_star_cells.cuh.
 //
 // Every mbarrier wait is bounded (GPW_ETIMEDOUT in the status word).

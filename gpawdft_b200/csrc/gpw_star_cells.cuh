@@ -21,9 +21,13 @@
 //    times, measured 9% slower for float64 and 4% faster for complex128.)
 // Measured against the kernel it replaced (one element a cell, its address
 // recomputed per plane, two barriers a plane), applies with a potential, R = 3:
-// 48 x 95^3 float64 238 -> 216 us, 48 x 96^3 complex128 549 -> 537 us, 64 x 84 x
-// 90 x 108 complex64 537 -> 423 us (3.0, 2.5 and 2.0 TB/s of compulsory bytes):
-// bound by shared-memory reads and, in single precision, issue slots.
+// 48 x 95^3 float64 238 -> 216 us, 48 x 96^3 complex128 549 -> 536 us, 64 x 84 x
+// 90 x 108 complex64 537 -> 423 us (3.0, 2.5 and 2.0 TB/s of compulsory bytes).
+// What bounds it: latency, at 14 - 15 warps per SM (128 registers) that wait for
+// shared memory and for their own arithmetic.  Of their rates complex128 uses
+// 40% of shared memory's, 42% of the issue slots, 24% of float64's, complex64 44%
+// and 50%; float64 on odd rows 56% and 45%, and 83% of the L1 with its one
+// cp.async per element.
 // Each output sums its terms in one fixed order (axis 0 below, centre and
 // axis 1 plus axis 2, axis 0 above), the order of gpw_rows.cuh and
 // gpw_star_tma.cuh.

@@ -1,8 +1,8 @@
 // TMA-fed star stencil for real grids with zero boundaries (sm_100a).
 //
 // The fast path of the Poisson V-cycle (every relax sweep and residual) and
-// of FD applies on 16-byte-pitched real grids.  Compared with the cp.async
-// kernel in gpw_stencil.cuh:
+// of FD applies on 16-byte-pitched real grids.  Compared with staging
+// cell by cell (gpw_star_cells.cuh):
 //  * one thread issues one 4D TMA tile load (cp.async.bulk.tensor) per plane
 //    into a ring of shared-memory stages, completing on an mbarrier; the
 //    tensor map's out-of-bounds zero fill *is* the zero boundary condition

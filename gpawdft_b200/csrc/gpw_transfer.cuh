@@ -14,8 +14,10 @@
 // pass evaluates the reference's expression in the reference's order with
 // unfused multiply / add, so results are bit-identical to the reference C.
 //
-// Bound by the unfused float64 multiplies and adds and the barrier of a step.
-// Two input planes a step and one barrier instead of one plane and a barrier
+// What bounds them (K = 6, float64): the restriction latency, at 15 warps per SM
+// with 63% of the shared-memory rate and 48% of the issue slots in use, the
+// interpolation issue (67%); the unfused arithmetic is 20% and 15% of float64's
+// rate.  Two input planes a step and one barrier instead of one plane and a barrier
 // per pass: K = 6, float64, restriction of 2 grids of 192^3 170 -> 59 us,
 // interpolation of 2 grids of 95^3 63.5 -> 51 us (with the caller's host work).
 //
@@ -204,8 +206,6 @@ __device__ __forceinline__ T interp_mid(const T* a, int st) {
 // the same two barriers, on two axis-2 buffers.  Of the 2K - 1 planes of an
 // output only the centre and the K at odd distance count, so a thread keeps
 // the last K even and K / 2 odd planes.
-// What bounds it: instruction issue and the float64 adds and multiplies of
-// the three unfused passes.
 template <typename T, int K>
 struct RestrictCfg {
   // tile of coarse points, one axis-1 item a thread; 16-byte elements of the

@@ -7,8 +7,8 @@ phase_cd)`` (c/operators.c:316-405) and ``Htpsit += psit * vt``
 restated operator over the compiled reference C (NumPy restatement where it
 is not built) and the NumPy product.  Every kernel that serves an apply
 carries the potential term -- the zero-boundary TMA star kernel, the
-periodic / Bloch row kernel (each tile layout pinned in turn), the cp.async
-star kernel and the general-offset kernel -- so each is pinned here.  Bars:
+periodic / Bloch row kernel (each tile layout pinned in turn), the cell-
+staged or direct star kernel and the general-offset kernel -- so each is pinned here.  Bars:
 1e-12 relative for float64 / complex128, 2e-6 for float32 / complex64.
 """
 import numpy as np
@@ -91,7 +91,7 @@ def test_zero_boundary_real(cuda, dtype):
 
 def test_cpasync_star_kernel(cuda):
     """Rows longer than the row kernel takes (130 complex points): the
-    cp.async star kernel."""
+    direct star kernel."""
     gd, ogd, kin, okin, psi, vt, ph = _setup((16, 20, 130), (3.2, 4.0, 26.0),
                                              1, complex, nb=2, seed=4)
     out = np.empty_like(psi)
