@@ -232,14 +232,12 @@ __global__ void __launch_bounds__(CellsCfg<T, R, MODE, TZ, CELLB, PY>::NT, (Cell
               if (j < rows) ep[j] = gload(q + j * eps1);
           }
         }
-        // plane p is one of this chunk's outputs (a halo plane has no potential
-        // of its own, and may lie outside the array)
-        const bool own = p >= z0 && p < z1;
         auto gpot = [&](int j, int e) {
           return j < rows && e < nx ? pot0[(int64_t)p * a.vout.s0 + j * a.vout.s1 + e] : S(0);
         };
+        // (a halo plane has no potential of its own, and may lie outside the array)
         if constexpr (EPI == 1) {
-          if (own) {
+          if (p >= z0 && p < z1) {
 #pragma unroll
             for (int j = 0; j < PY; ++j)
 #pragma unroll
@@ -317,7 +315,7 @@ __global__ void __launch_bounds__(CellsCfg<T, R, MODE, TZ, CELLB, PY>::NT, (Cell
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) part.v[e] = fma(pv[j][e / CS], c.v[e], part.v[e]);
               } else if constexpr (EPI == 2) {
-                if (pot0 && own) {
+                if (pot0 && p >= z0 && p < z1) {
 #pragma unroll
                   for (int e = 0; e < VEC; ++e) part.v[e] = fma(gpot(j, e / CS), c.v[e], part.v[e]);
                 }
