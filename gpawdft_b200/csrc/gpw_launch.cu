@@ -1252,10 +1252,11 @@ cudaError_t launch_transfer(const TrDesc& d, int dtype, const void* in, const Gr
   // every other K = 2 transfer of real data, and complex ones of little data
   // (input of a restriction, output of an interpolation) unless a test pins
   // their restriction kernel.  Time of the tile or row kernels over these, 400
-  // random grids: interpolations 1.07 up to 2 MB, 0.88 to 4, 0.6 - 0.8 above;
+  // random grids: interpolations of complex64 1.1 up to 2 MB, 0.88 to 4, 0.6 -
+  // 0.8 above, of complex128 1.06 up to 4, 0.88 to 8, 0.6 - 0.8 above;
   // restrictions of complex64 1.1 up to 8 MB, 0.98 to 16, 0.8 above, of
   // complex128 1.4 up to 8, 1.16 to 16, 0.85 above.
-  const int64_t most = interp ? 2 << 20 : (dtype == GPW_C128 ? 16 << 20 : 8 << 20);
+  const int64_t most = (dtype == GPW_C128 ? 2 : 1) * (interp ? 2LL << 20 : 8LL << 20);
   const bool small = direct_ok(interp ? vout : vin, nbatch, elt_size(dtype), most);
   if (d.k == 2 &&
       (dtype == GPW_F64 || dtype == GPW_F32 || (small && (interp || g_restrict_force.load() == 0)))) {
